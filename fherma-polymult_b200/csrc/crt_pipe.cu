@@ -27,20 +27,19 @@
 //   * the constant image (U x 128 bytes per chunk of 32 primes, the last chunk
 //     cut to the K steps it uses) is loaded once per CTA by bulk copies and
 //     stays resident in shared memory, so the MMAs never wait for constants;
-//   * warp 2 (one thread) streams y through a ring of 16 KB slots (as many as
-//     shared memory holds beside the constants, 2 to 6) with 2-D TMA copies:
-//     per chunk a box of 32 primes x 128 coefficients of the prime-major
-//     K x N array;
+//   * warp 1 (one thread) streams y through a ring of 16 KB boxes with 2-D TMA
+//     copies: per chunk a box of 32 primes x 128 coefficients of the
+//     prime-major K x N array;
 //   * warps 2-9, two threads per row (each half of a chunk's 32 primes), read
-//     their 16 values from the slot (conflict-free), meet at a named barrier,
-//     and write the same values back into that slot in the MMA's K-major,
-//     128-byte-swizzled byte layout (a box and an A operand are both 16 KB,
-//     so one ring serves both and every slot is a y box in flight while the
-//     MMAs need none); they also add up the rounding sum and the top limb,
-//     and in the last chunk the two halves pool their sums through shared
-//     memory and the first puts v in the row;
+//     their 16 values from the box (conflict-free), add up the rounding sum and
+//     the top limb, and write the values in the MMA's K-major,
+//     128-byte-swizzled byte layout to one of two operand slots.  Boxes and
+//     operands have rings of their own, so no warp waits for another's reads
+//     (writing over the box in place took a barrier of all eight warps per
+//     chunk).  In the last chunk the first half waits for the second half's
+//     sums of its 32 rows and puts v in the row;
 //   * warp 0 (one thread) issues a chunk's MMAs as soon as its slot holds A,
-//     and frees the slot for the next box when they finish;
+//     and frees the slot when they finish;
 //   * warps 10-13 and 14-17 are two epilogue groups, one per TMEM buffer, one
 //     thread per row: a quotient estimate e from the top TMEM columns (within
 //     one of floor(X / q)), then one pass from the bottom limb up that
@@ -52,8 +51,13 @@
 // shared memory at the start: read from the parameter bank inside the loops
 // (a few KB swept by every chunk and every limb) they made the stagers and
 // the epilogue several times slower.
-// The kernel is compiled for the common limb counts (L = 64, 55, 28, 8) and
-// once for any L.
+// One epilogue loop serves every limb count (B200, us per launch, before ->
+// after, a copy unrolled per limb count before): L = 4 at N = 65536 18.4 -> 8.6,
+// L = 16 22.3 -> 9.8, L = 32 at N = 2^18 106 -> 55, L = 55 at N = 65536
+// 32.9 -> 20.8 (rows that start off a 16-byte boundary now leave as 16-byte
+// stores too), L = 64 26.2 -> 25.6.  What bounds it is the latency of the
+// stagers and of the epilogue's chain, not memory (53 MB in 25.6 us at L = 64)
+// or the tensor cores.
 //
 // Every wait is bounded (DevPoint::wait_ns); a timeout raises an abort flag
 // that every role checks, the copy and MMA issuers wait out what they have in
@@ -79,28 +83,32 @@ constexpr int kEpiWarp0 = 10;             // warps 10-13 (group 0), 14-17 (group
 constexpr uint32_t kCrtTile = 128;        // coefficients per tile
 constexpr uint32_t kChunk = 32;           // K rows (primes) per chunk
 constexpr int kMaxSlots = 6;
-// A slot holds a y box, [32 primes][128 coefficients] u32, and then the A
-// operand made from it, 128 rows x 128 bytes, 128-byte swizzled.
+constexpr uint32_t kMaxASlots = 2;
+// A slot holds a y box, [32 primes][128 coefficients] u32, or the A operand
+// made from one, 128 rows x 128 bytes, 128-byte swizzled: the first ny slots
+// are boxes, the last na operands.
 constexpr uint32_t kSlot = kChunk * kCrtTile * 4;
-constexpr uint32_t kStagerBar = 1;        // named barrier of the 256 stager threads
-constexpr int kX = kMaxL + 2;
 constexpr size_t kSmemLimit = 227 * 1024;
 // Shared copies of the constants: {cf_j bits, top_j, sh_j, 0} per row
 // j < 32 nch (zero beyond the K + 1 rows), then q.
 constexpr size_t kConstBytes = (kMaxK + 1) * sizeof(uint4) + ((kMaxL + 2) * 4 + 15) / 16 * 16;
+
+constexpr int kBars = 34;
 
 // Shared-memory plan, the same on host and device: the resident constants
 // from 0, then the slot ring (1024-byte aligned), the per-tile top-limb words,
 // the constants and the barriers.
 struct Layout {
     uint32_t b_bytes;      // resident constant image
-    uint32_t slots;        // ring depth
+    uint32_t slots;        // of both rings
+    __host__ __device__ uint32_t na() const { return slots >= 4 ? kMaxASlots : 1u; }
+    __host__ __device__ uint32_t ny() const { return slots - na(); }
     __host__ __device__ size_t slot_off() const { return (size_t(b_bytes) + 1023) / 1024 * 1024; }
     __host__ __device__ size_t meta_off() const { return slot_off() + slots * size_t(kSlot); }
     __host__ __device__ size_t xch_off() const { return meta_off() + 2 * kCrtTile * sizeof(uint4); }
-    __host__ __device__ size_t const_off() const { return xch_off() + kCrtTile * sizeof(uint4); }
+    __host__ __device__ size_t const_off() const { return xch_off() + 2 * kCrtTile * sizeof(uint4); }
     __host__ __device__ size_t bar_off() const { return const_off() + kConstBytes; }
-    __host__ __device__ size_t bytes() const { return bar_off() + 32 * 8 + 16; }
+    __host__ __device__ size_t bytes() const { return bar_off() + kBars * 8 + 16; }
 };
 
 // Bytes of the constant image the MMAs read: full chunks of U x 128 bytes,
@@ -121,15 +129,18 @@ Layout make_layout(int K, uint32_t U) {
 
 struct Smem {
     uint8_t* b;          // resident constant image
-    uint8_t* slot;       // [slots][kSlot]
+    uint8_t* slot;       // [ny][kSlot] y boxes
+    uint8_t* aop;        // [na][kSlot] A operands
     uint4* meta;         // [2][128] {top-limb words 0, 1, 2, -}
-    uint4* xch;          // [128] second halves' sums {rounding sum, top-limb words 0, 1, 2}
+    uint4* xch;          // [2][128] second halves' sums {rounding sum, top-limb words 0, 1, 2}
     uint4* kc;           // [kMaxK + 1] {cf_j bits, top_j, sh_j, 0}
     uint32_t* qs;        // [L + 2] q, zero above L
     uint64_t* b_full;    // [1] the constant image landed
     uint64_t* y_full;    // [kMaxSlots] the slot's TMA box landed
-    uint64_t* a_full;    // [kMaxSlots] 128 rows of A staged in it
-    uint64_t* s_empty;   // [kMaxSlots] its MMAs finished
+    uint64_t* y_empty;   // [kMaxSlots] and the stagers have read it
+    uint64_t* a_full;    // [kMaxASlots] 128 rows of A staged
+    uint64_t* a_empty;   // [kMaxASlots] and its MMAs finished
+    uint64_t* x_full;    // [4][2] the second halves' sums of 32 rows are in xch
     uint64_t* d_full;    // [2] a tile's MMAs finished (per TMEM buffer)
     uint64_t* d_empty;   // [2] its epilogue group has read TMEM
     uint64_t* m_full;    // [2] a tile's top-limb words staged
@@ -142,6 +153,7 @@ __device__ inline Smem carve(uint8_t* base, const Layout& lay) {
     Smem s;
     s.b = base;
     s.slot = base + lay.slot_off();
+    s.aop = s.slot + lay.ny() * kSlot;
     s.meta = reinterpret_cast<uint4*>(base + lay.meta_off());
     s.xch = reinterpret_cast<uint4*>(base + lay.xch_off());
     s.kc = reinterpret_cast<uint4*>(base + lay.const_off());
@@ -149,29 +161,28 @@ __device__ inline Smem carve(uint8_t* base, const Layout& lay) {
     uint64_t* bars = reinterpret_cast<uint64_t*>(base + lay.bar_off());
     s.b_full = bars;
     s.y_full = bars + 1;
-    s.a_full = bars + 1 + kMaxSlots;
-    s.s_empty = bars + 1 + 2 * kMaxSlots;
-    s.d_full = bars + 1 + 3 * kMaxSlots;
+    s.y_empty = s.y_full + kMaxSlots;
+    s.a_full = s.y_empty + kMaxSlots;
+    s.a_empty = s.a_full + kMaxASlots;
+    s.x_full = s.a_empty + kMaxASlots;
+    s.d_full = s.x_full + 8;
     s.d_empty = s.d_full + 2;
     s.m_full = s.d_full + 4;
     s.m_empty = s.d_full + 6;
-    s.tmem_base = reinterpret_cast<uint32_t*>(bars + 32);
+    s.tmem_base = reinterpret_cast<uint32_t*>(bars + kBars);
     s.abort = s.tmem_base + 1;
     return s;
 }
 
-static_assert(1 + 3 * kMaxSlots + 8 <= 32, "barriers fit before tmem_base");
+static_assert(1 + 2 * kMaxSlots + 2 * kMaxASlots + 8 + 8 <= kBars, "barriers fit before tmem_base");
 
-// bar.red.and over the 256 stager threads: true when every one passed true.
-// All of them reach it whatever their outcome, so none can be left waiting.
-__device__ __forceinline__ bool stagers_all(bool p) {
-    uint32_t r;
-    asm volatile(
-        "{ .reg .pred pi, po; setp.ne.u32 pi, %1, 0; bar.red.and.pred po, %2, %3, pi; selp.u32 %0, 1, 0, po; }"
-        : "=r"(r)
-        : "r"(static_cast<uint32_t>(p)), "n"(kStagerBar), "n"(kStagers)
-        : "memory");
-    return r != 0;
+// A shared load that the compiler may neither repeat nor move past the
+// barrier arrival that hands the slot back (a plain load may be done again
+// later instead of keeping its register, when TMA has refilled the slot).
+__device__ __forceinline__ uint32_t ld_shared_once(uint32_t addr) {
+    uint32_t x;
+    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(x) : "r"(addr) : "memory");
+    return x;
 }
 
 // Waits for this thread's TMEM loads; naming the registers keeps every read of
@@ -185,8 +196,112 @@ __device__ __forceinline__ void tmem_wait(uint32_t (&r)[16]) {
                  : "memory");
 }
 
-// LT > 0: L = LT at compile time; LT = 0: any L (predicated).
-template <int LT>
+// The carry chain of one row from the bottom limb up.  X = Z0 + 2^8 Z1 +
+// 2^16 Z2 + 2^24 Z3, Z_s the number whose limb l is D[4 l + s] (< 2^26), so
+// limb l of 2^(8 s) Z_s is one funnel shift of Z_s[l - 1] and Z_s[l] and the
+// limb's share of X is z0 + s1 + s2 + s3 < 2^34 with no products.  e q's words
+// come from a running sum, two multiply-adds a limb: what is carried is below
+// 2^33, e_lo q_l below (2^32 - 1)^2 and e_hi q_(l-1) below 2^38, so the sum
+// never wraps.  The carry chain itself is one signed 64-bit add a limb.
+struct LimbChain {
+    uint32_t e_lo, e_hi;
+    uint64_t eq = 0;     // e q from this limb's word up, the limbs below it added
+    uint32_t qp = 0;
+    uint32_t z1p = 0, z2p = 0, z3p = 0;
+    int64_t cy = 0;
+    __device__ __forceinline__ LimbChain(uint32_t lo, uint32_t hi) : e_lo(lo), e_hi(hi) {}
+    // extra: what the limb gets besides its columns (a top-limb word).
+    __device__ __forceinline__ uint32_t limb(uint32_t z0, uint32_t z1, uint32_t z2, uint32_t z3, uint32_t extra,
+                                             uint32_t qk) {
+        const uint64_t sd = static_cast<uint64_t>(z0) + __funnelshift_l(z1p, z1, 8) +
+                            static_cast<uint64_t>(__funnelshift_l(z2p, z2, 16)) + __funnelshift_l(z3p, z3, 24) + extra;
+        z1p = z1;
+        z2p = z2;
+        z3p = z3;
+        eq = static_cast<uint64_t>(e_lo) * qk + (eq >> 32);
+        eq += static_cast<uint64_t>(e_hi) * qp;
+        qp = qk;
+        const int64_t v = static_cast<int64_t>(sd) - static_cast<int64_t>(static_cast<uint32_t>(eq)) + cy;
+        cy = v >> 32;
+        return static_cast<uint32_t>(v);
+    }
+    // Four limbs below limb L - 1.
+    __device__ __forceinline__ void piece(const uint32_t (&z)[16], const uint32_t* q, uint32_t (&o)[4]) {
+        const uint4 q4 = *reinterpret_cast<const uint4*>(q);
+        o[0] = limb(z[0], z[1], z[2], z[3], 0u, q4.x);
+        o[1] = limb(z[4], z[5], z[6], z[7], 0u, q4.y);
+        o[2] = limb(z[8], z[9], z[10], z[11], 0u, q4.z);
+        o[3] = limb(z[12], z[13], z[14], z[15], 0u, q4.w);
+    }
+};
+
+// 2^n exactly, |n| < 1000.
+__device__ __forceinline__ double pow2(int n) { return __hiloint2double((1023 + n) << 20, 0); }
+
+// Stores a row's limbs four at a time as aligned 16-byte words: a row starts
+// r = 0 .. 3 words past a 16-byte boundary (rows of L words, any L and any
+// base), so aligned group g holds limbs 4 g - r .. 4 g - r + 3, the last r of
+// piece g - 1 and the first 4 - r of piece g.
+template <bool EVEN>
+struct RowStore {
+    uint32_t* base;      // the row, rounded down to 16 bytes
+    uint32_t r;
+    bool live;
+    uint32_t prev[4] = {};
+    __device__ __forceinline__ RowStore(uint32_t* row, bool on)
+        : base(row - ((reinterpret_cast<uintptr_t>(row) >> 2) & 3u)),
+          r(static_cast<uint32_t>(reinterpret_cast<uintptr_t>(row) >> 2) & 3u),
+          live(on) {}
+    __device__ __forceinline__ void piece(const uint32_t (&o)[4], int g) {
+        if constexpr (EVEN) {
+            if (live) *reinterpret_cast<uint4*>(base + 4 * g) = make_uint4(o[0], o[1], o[2], o[3]);
+            return;
+        }
+        const bool r1 = (r & 1u) != 0, r2 = (r & 2u) != 0;
+        // t[i + 2]: the word i places from the piece's start, moved by r & 1.
+        uint32_t t[6];
+        t[0] = r1 ? prev[1] : prev[2];
+        t[1] = r1 ? prev[2] : prev[3];
+        t[2] = r1 ? prev[3] : o[0];
+        t[3] = r1 ? o[0] : o[1];
+        t[4] = r1 ? o[1] : o[2];
+        t[5] = r1 ? o[2] : o[3];
+        uint32_t* at = base + 4 * g;
+        const uint4 v = make_uint4(r2 ? t[0] : t[2], r2 ? t[1] : t[3], r2 ? t[2] : t[4], r2 ? t[3] : t[5]);
+        if (live) {
+            if (g > 0 || r == 0) {
+                *reinterpret_cast<uint4*>(at) = v;
+            } else {
+                // The first r words belong to the row before.
+                if (r < 2) at[1] = v.y;
+                if (r < 3) at[2] = v.z;
+                at[3] = v.w;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) prev[i] = o[i];
+    }
+    // After piece g - 1: its last r words, which no aligned group has taken.
+    __device__ __forceinline__ void flush(int g) {
+        if (!EVEN && live && g > 0) {
+            uint32_t* at = base + 4 * g;
+            if (r == 1) {
+                at[0] = prev[3];
+            } else if (r == 2) {
+                at[0] = prev[2];
+                at[1] = prev[3];
+            } else if (r == 3) {
+                at[0] = prev[1];
+                at[1] = prev[2];
+                at[2] = prev[3];
+            }
+        }
+    }
+};
+
+// EVEN: every row of C starts on a 16-byte boundary (L a multiple of 4, C
+// aligned), so a piece of four limbs is one store.
+template <bool EVEN>
 __global__ void __launch_bounds__(kThreads, 1)
     k_crt_pipe(DevPoint d, const __grid_constant__ CrtConsts cc, const __grid_constant__ CUtensorMap tmY,
                uint32_t* __restrict__ C, uint32_t n_begin, uint32_t n_end, Layout lay) {
@@ -200,12 +315,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     const Smem sm = carve(smem_raw, lay);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int L = LT > 0 ? LT : d.L;
+    const int L = d.L;
     const int K = d.K;
-    const uint32_t U = LT > 0 ? (4 * LT - 1 + 31) / 32 * 32 : d.crt_u;
+    const uint32_t U = d.crt_u;
     const int nch = (K + 1 + static_cast<int>(kChunk) - 1) / static_cast<int>(kChunk);   // K + 1 rows
     const uint32_t tiles = (n_end - n_begin + kCrtTile - 1) / kCrtTile;
-    const uint32_t ns = lay.slots;
+    const uint32_t ny = lay.ny(), na = lay.na();
     const uint64_t lim = d.wait_ns;
 
     if (threadIdx.x == 0) {
@@ -216,11 +331,15 @@ __global__ void __launch_bounds__(kThreads, 1)
             tc::mbar_init(&sm.m_full[i], kCrtTile);
             tc::mbar_init(&sm.m_empty[i], kCrtTile);
         }
-        for (uint32_t i = 0; i < ns; ++i) {
+        for (uint32_t i = 0; i < ny; ++i) {
             tc::mbar_init(&sm.y_full[i], 1);
-            tc::mbar_init(&sm.a_full[i], kStagers);
-            tc::mbar_init(&sm.s_empty[i], 1);
+            tc::mbar_init(&sm.y_empty[i], kStagers);
         }
+        for (uint32_t i = 0; i < na; ++i) {
+            tc::mbar_init(&sm.a_full[i], kStagers);
+            tc::mbar_init(&sm.a_empty[i], 1);
+        }
+        for (int i = 0; i < 8; ++i) tc::mbar_init(&sm.x_full[i], 32);
         *sm.abort = 0;
         tc::fence_mbar_init();
         // The constant image is read-only plan data: it loads under the
@@ -256,15 +375,15 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (uint32_t t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
                 const int x = static_cast<int>(n_begin + t * kCrtTile);
                 for (int c = 0; c < nch; ++c, ++g) {
-                    const uint32_t s = g % ns, u = g / ns;
-                    if (u >= 1 && !(ok = tc::wait_or_abort(&sm.s_empty[s], (u - 1) & 1, sm.abort, lim))) break;
+                    const uint32_t s = g % ny, u = g / ny;
+                    if (u >= 1 && !(ok = tc::wait_or_abort(&sm.y_empty[s], (u - 1) & 1, sm.abort, lim))) break;
                     tc::mbar_arrive_expect_tx(&sm.y_full[s], kSlot);
                     tc::tma_load_2d(sm.slot + s * kSlot, &tmY, x, c * static_cast<int>(kChunk), &sm.y_full[s]);
                     par[s] = u & 1;
                     armed[s] = true;
                 }
             }
-            for (uint32_t s = 0; s < ns; ++s) {
+            for (uint32_t s = 0; s < ny; ++s) {
                 if (armed[s]) tc::wait_parity(&sm.y_full[s], par[s], lim);
             }
         }
@@ -281,12 +400,12 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const uint32_t buf = i & 1, use = i >> 1;
                 if (use >= 1 && !(ok = tc::wait_or_abort(&sm.d_empty[buf], (use - 1) & 1, sm.abort, lim))) break;
                 for (int c = 0; c < nch; ++c, ++g) {
-                    const uint32_t s = g % ns;
-                    const uint32_t ph = (g / ns) & 1;
+                    const uint32_t s = g % na;
+                    const uint32_t ph = (g / na) & 1;
                     ok = tc::wait_or_abort(&sm.a_full[s], ph, sm.abort, lim);
                     if (!ok) break;
                     tc::tc_fence_after();
-                    const uint32_t a0 = tc::smem_addr(sm.slot + s * kSlot), b0 = tc::smem_addr(sm.b + c * U * 128);
+                    const uint32_t a0 = tc::smem_addr(sm.aop + s * kSlot), b0 = tc::smem_addr(sm.b + c * U * 128);
                     // K steps of 8 rows; the last chunk stops after row K.
                     const int rows_c = min(static_cast<int>(kChunk), K + 1 - c * static_cast<int>(kChunk));
                     const uint32_t ksteps = static_cast<uint32_t>(rows_c + 7) / 8;
@@ -300,8 +419,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                                                   : tc::smem_desc(b0 + kk * 2 * (U * 16), U * 16, 128);
                         tc::mma_u8(tmem + buf * 256, ad, bd, idesc, c > 0 || kk > 0);
                     }
-                    tc::mma_commit(&sm.s_empty[s]);
-                    last_bar = &sm.s_empty[s];
+                    tc::mma_commit(&sm.a_empty[s]);
+                    last_bar = &sm.a_empty[s];
                     last_par = ph;
                 }
                 if (!ok) break;
@@ -319,10 +438,13 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t st = threadIdx.x - kStagerWarp0 * 32;
         const uint32_t m = st & (kCrtTile - 1), h = st / kCrtTile;
         constexpr int kHalf = static_cast<int>(kChunk) / 2;
+        const uint32_t rw = m >> 5;   // the warp pair (halves 0 and 1) of these 32 rows
         uint32_t g = 0, i = 0;
+        uint32_t ys = 0, yph = 0, as_ = 0, aph = 0;   // ring positions of chunk g and their phases
         for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x, ++i) {
             const uint32_t n0 = n_begin + t * kCrtTile;
             const bool live = m < min(kCrtTile, n_end - n0);
+            const uint32_t xb = i & 1;
             // The rounding sum as kPart float partial sums; the top-limb sum
             // sum_j y_j top_j (< 2^71) as 96 bits (t01, t2), fed by 64-bit
             // pairs of products (each < 2^63 with 31-bit primes, so a pair
@@ -335,18 +457,12 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll 1
             for (int c = 0; c < nch; ++c) {
                 uint32_t yv[kHalf];
-                const uint32_t s = g % ns;
-                ok = tc::wait_or_abort(&sm.y_full[s], (g / ns) & 1, sm.abort, lim);
+                ok = tc::wait_or_abort(&sm.y_full[ys], yph, sm.abort, lim);
                 ok = __all_sync(0xffffffffu, ok);
-                if (ok) {
-                    const uint32_t* yrow = reinterpret_cast<const uint32_t*>(sm.slot + s * kSlot) + h * kHalf * kCrtTile + m;
-#pragma unroll
-                    for (int jj = 0; jj < kHalf; ++jj) yv[jj] = yrow[jj * kCrtTile];
-                }
-                // Every row has read the box before any writes A over it (and
-                // the eight warps leave together on an abort).
-                ok = stagers_all(ok);
                 if (!ok) break;
+                const uint32_t yrow = tc::smem_addr(sm.slot + ys * kSlot) + 4 * (h * kHalf * kCrtTile + m);
+#pragma unroll
+                for (int jj = 0; jj < kHalf; ++jj) yv[jj] = ld_shared_once(yrow + 4 * jj * kCrtTile);
                 // Rows j >= K of the box read as zero and cf_j = 0 there, so
                 // every row of the chunk takes part without a test.
                 const uint4* kc = sm.kc + c * static_cast<int>(kChunk) + h * kHalf;
@@ -363,65 +479,70 @@ __global__ void __launch_bounds__(kThreads, 1)
                     t01 += grp;
                     t2 += t01 < grp ? 1u : 0u;
                 }
+                // Every value has been used, so its load is done: the box goes
+                // back (the fence orders these reads before the TMA's writes).
+                tc::fence_proxy_async_smem();
+                tc::mbar_arrive(&sm.y_empty[ys]);
+                if (++ys == ny) ys = 0, yph ^= 1;
+                // The operand slot is free once the MMAs of chunk g - na are done.
+                if (g >= na) {
+                    ok = tc::wait_or_abort(&sm.a_empty[as_], aph ^ 1, sm.abort, lim);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                }
                 // Row m's 128 bytes in the 128-byte-swizzle layout
                 // (sw128_offset); this half owns 16-byte pieces 4 h .. 4 h + 3.
-                uint8_t* as = sm.slot + s * kSlot + m * 128;
+                uint8_t* as = sm.aop + as_ * kSlot + m * 128;
                 const bool last = c == nch - 1;
-                if (last) {
+                if (last && h == 0) {
                     // Row K: the multiplier v of -P mod q, from both halves'
-                    // sums; the first half writes it (and its own pieces) once
-                    // the second has written its pieces and sums.
+                    // sums, once the second half has written its pieces and
+                    // sums (xch[xb] is rewritten two tiles on, at least two
+                    // chunks: not before this chunk's MMAs).
+                    ok = tc::wait_or_abort(&sm.x_full[2 * rw + xb], (i >> 1) & 1, sm.abort, lim);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
                     const float vh = (vf[0] + vf[1]) + (vf[2] + vf[3]);
-                    if (h == 1) {
+                    const uint4 x = sm.xch[xb * kCrtTile + m];
+                    int v = __float2int_rn((vh + __uint_as_float(x.x)) - cc.voff);
+                    v = v < 0 ? 0 : (v > K ? K : v);
+                    const uint32_t vu = live ? static_cast<uint32_t>(v) : 0u;
+                    const uint64_t other = (static_cast<uint64_t>(x.z) << 32) | x.y;
+                    t01 += other;
+                    t2 += x.w + (t01 < other ? 1u : 0u);
+                    const uint64_t pv = static_cast<uint64_t>(vu) * sm.kc[K].y;
+                    t01 += pv;
+                    t2 += t01 < pv ? 1u : 0u;
+                    const uint32_t kk = static_cast<uint32_t>(K) % kChunk;
 #pragma unroll
-                        for (int q4 = 0; q4 < 4; ++q4)
-                            *reinterpret_cast<uint4*>(as + (((4 + q4) ^ (m & 7)) << 4)) =
-                                make_uint4(yv[4 * q4], yv[4 * q4 + 1], yv[4 * q4 + 2], yv[4 * q4 + 3]);
-                        sm.xch[m] = make_uint4(__float_as_uint(vh), static_cast<uint32_t>(t01),
-                                               static_cast<uint32_t>(t01 >> 32), t2);
-                    }
-                    stagers_all(true);
-                    if (h == 0) {
-                        const uint4 x = sm.xch[m];
-                        int v = __float2int_rn((vh + __uint_as_float(x.x)) - cc.voff);
-                        v = v < 0 ? 0 : (v > K ? K : v);
-                        const uint32_t vu = live ? static_cast<uint32_t>(v) : 0u;
-                        const uint64_t other = (static_cast<uint64_t>(x.z) << 32) | x.y;
-                        t01 += other;
-                        t2 += x.w + (t01 < other ? 1u : 0u);
-                        const uint64_t pv = static_cast<uint64_t>(vu) * sm.kc[K].y;
-                        t01 += pv;
-                        t2 += t01 < pv ? 1u : 0u;
-                        const uint32_t kk = static_cast<uint32_t>(K) % kChunk;
+                    for (int jj = 0; jj < kHalf; ++jj)
+                        if (static_cast<uint32_t>(jj) == kk) yv[jj] = vu;
+                    if (kk >= static_cast<uint32_t>(kHalf))
+                        *reinterpret_cast<uint32_t*>(as + (((kk >> 2) ^ (m & 7)) << 4) + 4 * (kk & 3)) = vu;
+                }
 #pragma unroll
-                        for (int jj = 0; jj < kHalf; ++jj)
-                            if (static_cast<uint32_t>(jj) == kk) yv[jj] = vu;
-#pragma unroll
-                        for (int q4 = 0; q4 < 4; ++q4)
-                            *reinterpret_cast<uint4*>(as + ((q4 ^ (m & 7)) << 4)) =
-                                make_uint4(yv[4 * q4], yv[4 * q4 + 1], yv[4 * q4 + 2], yv[4 * q4 + 3]);
-                        if (kk >= static_cast<uint32_t>(kHalf))
-                            *reinterpret_cast<uint32_t*>(as + (((kk >> 2) ^ (m & 7)) << 4) + 4 * (kk & 3)) = vu;
-                    }
-                } else {
-#pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4)
-                        *reinterpret_cast<uint4*>(as + (((4 * h + q4) ^ (m & 7)) << 4)) =
-                            make_uint4(yv[4 * q4], yv[4 * q4 + 1], yv[4 * q4 + 2], yv[4 * q4 + 3]);
+                for (int q4 = 0; q4 < 4; ++q4)
+                    *reinterpret_cast<uint4*>(as + (((4 * h + q4) ^ (m & 7)) << 4)) =
+                        make_uint4(yv[4 * q4], yv[4 * q4 + 1], yv[4 * q4 + 2], yv[4 * q4 + 3]);
+                if (last && h == 1) {
+                    const float vh = (vf[0] + vf[1]) + (vf[2] + vf[3]);
+                    sm.xch[xb * kCrtTile + m] = make_uint4(__float_as_uint(vh), static_cast<uint32_t>(t01),
+                                                           static_cast<uint32_t>(t01 >> 32), t2);
+                    tc::mbar_arrive(&sm.x_full[2 * rw + xb]);
                 }
                 tc::fence_proxy_async_smem();
-                tc::mbar_arrive(&sm.a_full[s]);
+                tc::mbar_arrive(&sm.a_full[as_]);
+                if (++as_ == na) as_ = 0, aph ^= 1;
                 ++g;
             }
             if (!ok) break;
-            const int p = i & 1;
-            if (h == 0 && i >= 2) {
-                ok = tc::wait_or_abort(&sm.m_empty[p], ((i - 2) >> 1) & 1, sm.abort, lim);
-                ok = __all_sync(0xffffffffu, ok);
-            }
-            ok = stagers_all(ok);
-            if (!ok) break;
             if (h == 0) {
+                const int p = i & 1;
+                if (i >= 2) {
+                    ok = tc::wait_or_abort(&sm.m_empty[p], ((i - 2) >> 1) & 1, sm.abort, lim);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                }
                 // Top-limb sum as three words.
                 sm.meta[p * kCrtTile + m] =
                     make_uint4(static_cast<uint32_t>(t01), static_cast<uint32_t>(t01 >> 32), t2, 0u);
@@ -434,18 +555,18 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t grp = static_cast<uint32_t>(warp - kEpiWarp0) >> 2, qd = warp & 3;
         const uint32_t row = qd * 32 + lane;
         const uint32_t tq = tmem + ((qd * 32) << 16) + grp * 256;
-        const uint32_t npieces = U / 16;
-        const int n = L + 2, drop = top_drop(L);
-        const uint32_t top_piece = static_cast<uint32_t>(4 * drop) / 16;
-        const bool gvec = (L & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;   // 16-byte row stores
-        constexpr int kXL = LT > 0 ? LT + 2 : kX;        // limbs handled
-        constexpr int kPieces = (kXL + 3) / 4;
+        const int drop = top_drop(L);
+        const int tail = (L - 1) / 4;                    // the piece (four limbs, 16 columns) of limb L - 1
+        const int top_piece = drop / 4;
+        const double piece_w = pow2(32 * (4 * top_piece - drop)), top_w = pow2(32 * (L - 1 - drop));
+        const bool spill = static_cast<uint32_t>(tail + 1) * 16 < U;   // the piece above `tail` has columns
         uint32_t k = 0;   // this group's tiles so far
         for (uint32_t t = blockIdx.x + grp * gridDim.x; t < tiles; t += 2 * gridDim.x, ++k) {
             const uint32_t n0 = n_begin + t * kCrtTile;
             const uint32_t rows_t = min(kCrtTile, n_end - n0);
             const bool live = row < rows_t;
             uint32_t* crow = C + static_cast<size_t>(n0 + (live ? row : 0)) * L;
+            RowStore<EVEN> out(crow, live);
             bool ok = tc::wait_or_abort(&sm.m_full[grp], k & 1, sm.abort, lim);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
@@ -456,89 +577,94 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (!ok) break;
             tc::tc_fence_after();
             uint32_t ra[16], rb[16];
-            // Quotient estimate from the columns at and above limb `drop` and the
-            // top-limb words: |estimate - X / q| < 2^-11, so e is within one.
+            // Quotient estimate from the limbs at and above `drop` (columns
+            // past limb L - 1 are zero) and the top-limb words:
+            // |estimate - X / q| < 2^-11, so e is within one.  A limb's four
+            // columns add up exactly in 64 bits before the conversion.
             double xd = 0;
-            for (uint32_t pc = npieces; pc-- > top_piece;) {
+            for (int pc = tail; pc >= top_piece; --pc) {
                 tc::tmem_ld16(tq + pc * 16, ra);
                 tmem_wait(ra);
 #pragma unroll
-                for (int kk = 15; kk >= 0; --kk) xd = xd * 256.0 + ra[kk];
+                for (int ii = 3; ii >= 0; --ii) {
+                    const uint64_t z = ra[4 * ii] + (static_cast<uint64_t>(ra[4 * ii + 1]) << 8) +
+                                       (static_cast<uint64_t>(ra[4 * ii + 2]) << 16) +
+                                       (static_cast<uint64_t>(ra[4 * ii + 3]) << 24);
+                    xd = xd * 4294967296.0 + static_cast<double>(z);
+                }
             }
-            xd = ldexp(xd, static_cast<int>(8 * 16 * top_piece) - 32 * drop) +
-                 ldexp(static_cast<double>(meta.x), 32 * (L - 1 - drop)) +
-                 ldexp(static_cast<double>(meta.y), 32 * (L - drop)) +
-                 ldexp(static_cast<double>(meta.z), 32 * (L + 1 - drop));
+            tc::tmem_ld16(tq, ra);
+            // (meta.x is limb L - 1's, meta.y and meta.z the two above it.)
+            xd = xd * piece_w + ((static_cast<double>(meta.z) * 4294967296.0 + static_cast<double>(meta.y)) * 4294967296.0 +
+                                 static_cast<double>(meta.x)) * top_w;
             const double fq = xd * d.q_top_inv;
             const double f = floor(fq);
             const uint64_t e = f > 0 ? static_cast<uint64_t>(f) : 0;
-            const uint32_t e_lo = static_cast<uint32_t>(e), e_hi = static_cast<uint32_t>(e >> 32);
             // With the fraction of the estimate at least 2^-8 from an integer,
             // e = floor(X / q) exactly and X - e q lies in [0, q); otherwise it
             // lies in [-q, 2q) and the row is checked after the pass.
             const double frac = fq - f;
             const bool near = !(frac >= 0x1p-8 && frac <= 1.0 - 0x1p-8);
-            // One pass from the bottom.  X = Z0 + 2^8 Z1 + 2^16 Z2 + 2^24 Z3,
-            // Z_s the number whose limb l is D[4 l + s] (< 2^26), so limb l of
-            // 2^(8 s) Z_s is one funnel shift of Z_s[l - 1] and Z_s[l] and the
-            // limb's share of X is z0 + s1 + s2 + s3 < 2^34 with no products.
-            // e q enters as words: lo(e_lo q_l) + hi(e_lo q_(l-1)) +
-            // lo(e_hi q_(l-1)) + hi(e_hi q_(l-2)).  Both are formed off the
-            // carry chain; the chain itself is one signed 64-bit add a limb.
-            // TMEM pieces are double-buffered: piece pc + 1 loads while piece
-            // pc is used.
-            uint64_t pp = 0, hp = 0, hp2 = 0;
-            uint32_t z1p = 0, z2p = 0, z3p = 0;
-            int64_t cy = 0;
-            uint32_t o[4], over = 0;
-            tc::tmem_ld16(tq, ra);
+            // One pass from the bottom, one loop for every L: unrolled over
+            // the 66 limbs of the widest modulus (as it was, but for four
+            // common L) the code alone cost a small product 6 us of
+            // instruction fetch.  TMEM pieces are double-buffered: piece
+            // pc + 1 loads while piece pc is used.
+            LimbChain ch(static_cast<uint32_t>(e), static_cast<uint32_t>(e >> 32));
+            uint32_t o[4];
             tmem_wait(ra);
+            int pc = 0;
+#pragma unroll 1
+            for (; pc + 2 <= tail; pc += 2) {
+                tc::tmem_ld16(tq + (pc + 1) * 16, rb);
+                ch.piece(ra, sm.qs + 4 * pc, o);
+                out.piece(o, pc);
+                tmem_wait(rb);
+                tc::tmem_ld16(tq + (pc + 2) * 16, ra);
+                ch.piece(rb, sm.qs + 4 * pc + 4, o);
+                out.piece(o, pc + 1);
+                tmem_wait(ra);
+            }
+            if (pc < tail) {
+                tc::tmem_ld16(tq + (pc + 1) * 16, rb);
+                ch.piece(ra, sm.qs + 4 * pc, o);
+                out.piece(o, pc);
+                tmem_wait(rb);
 #pragma unroll
-            for (int pc = 0; pc < kPieces; ++pc) {
-                uint32_t(&cur)[16] = (pc & 1) ? rb : ra;
-                uint32_t(&nxt)[16] = (pc & 1) ? ra : rb;
-                const bool have = static_cast<uint32_t>(pc) < npieces;
-                const bool more = static_cast<uint32_t>(pc + 1) < npieces;
-                if (more) tc::tmem_ld16(tq + (pc + 1) * 16, nxt);
+                for (int ii = 0; ii < 16; ++ii) ra[ii] = rb[ii];
+            }
+            // Limbs 4 tail .. L + 1: the last one to four of the result, with
+            // the top-limb words, and what lies above it.
 #pragma unroll
-                for (int ii = 0; ii < 4; ++ii) {
-                    const int kl = 4 * pc + ii;
-                    if (kl < kXL && kl < n) {
-                        const uint32_t z0 = have ? cur[4 * ii] : 0u, z1 = have ? cur[4 * ii + 1] : 0u;
-                        const uint32_t z2 = have ? cur[4 * ii + 2] : 0u, z3 = have ? cur[4 * ii + 3] : 0u;
-                        uint64_t sd = static_cast<uint64_t>(z0) + __funnelshift_l(z1p, z1, 8) +
-                                      static_cast<uint64_t>(__funnelshift_l(z2p, z2, 16)) + __funnelshift_l(z3p, z3, 24);
-                        z1p = z1;
-                        z2p = z2;
-                        z3p = z3;
-                        if (kl == L - 1) sd += meta.x;
-                        if (kl == L) sd += meta.y;
-                        if (kl == L + 1) sd += meta.z;
-                        const uint32_t qk = sm.qs[kl];
-                        const uint64_t P = static_cast<uint64_t>(e_lo) * qk, H = static_cast<uint64_t>(e_hi) * qk;
-                        const uint64_t t = (P & 0xFFFFFFFFu) + (pp >> 32) + (hp & 0xFFFFFFFFu) + (hp2 >> 32);
-                        pp = P;
-                        hp2 = hp;
-                        hp = H;
-                        const int64_t v = static_cast<int64_t>(sd) - static_cast<int64_t>(t) + cy;
-                        cy = v >> 32;
-                        const uint32_t yk = static_cast<uint32_t>(v);
-                        o[ii] = yk;
-                        if (kl < L) {
-                            if (live) {
-                                if (gvec) {
-                                    if (ii == 3) *reinterpret_cast<uint4*>(crow + kl - 3) = make_uint4(o[0], o[1], o[2], o[3]);
-                                } else {
-                                    crow[kl] = yk;
-                                }
-                            }
-                        } else {
-                            over |= yk;   // limbs L and L + 1 of a non-negative result
+            for (int ii = 0; ii < 16; ++ii) rb[ii] = 0;
+            if (spill) {
+                tc::tmem_ld16(tq + (tail + 1) * 16, rb);
+                tmem_wait(rb);
+            }
+            uint32_t over = 0;
+            out.flush(tail);
+#pragma unroll
+            for (int ii = 0; ii < 6; ++ii) {
+                const int kl = 4 * tail + ii;
+                if (EVEN || kl < L + 2) {
+                    const uint32_t(&z)[16] = ii < 4 ? ra : rb;
+                    const uint32_t x = EVEN ? (ii == 3 ? meta.x : ii == 4 ? meta.y : ii == 5 ? meta.z : 0u)
+                                            : (kl == L - 1 ? meta.x : kl == L ? meta.y : kl == L + 1 ? meta.z : 0u);
+                    const uint32_t y = ch.limb(z[4 * (ii & 3)], z[4 * (ii & 3) + 1], z[4 * (ii & 3) + 2],
+                                               z[4 * (ii & 3) + 3], x, sm.qs[kl]);
+                    if (EVEN ? ii < 4 : kl < L) {
+                        o[ii & 3] = y;
+                        if (EVEN) {
+                            if (ii == 3) out.piece(o, tail);
+                        } else if (live) {
+                            crow[kl] = y;
                         }
+                    } else {
+                        over |= y;   // limbs L and L + 1 of a non-negative result
                     }
                 }
-                if (more) tmem_wait(nxt);
             }
+            const int64_t cy = ch.cy;
             // TMEM is read: the MMAs of this buffer's next tile may start.
             tc::tc_fence_before();
             tc::mbar_arrive(&sm.d_empty[grp]);
@@ -584,13 +710,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
 }
 
-template <int LT>
-void set_attr() {
-    check(cudaFuncSetAttribute(k_crt_pipe<LT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(kSmemLimit)),
-          "crt_pipe smem");
-}
-
 }  // namespace
 
 CrtConsts make_crt_consts(const HostPlan& pl, const uint32_t* top) {
@@ -630,11 +749,9 @@ bool crt_pipe_supported(const DevPoint& d, const CrtConsts& cc, const uint32_t* 
 }
 
 void crt_pipe_init_attributes() {
-    set_attr<0>();
-    set_attr<64>();
-    set_attr<55>();
-    set_attr<28>();
-    set_attr<8>();
+    for (auto kernel : {k_crt_pipe<true>, k_crt_pipe<false>})
+        check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemLimit)),
+              "crt_pipe smem");
 }
 
 void launch_crt_pipe(const DevPoint& d, const CrtConsts& cc, const uint32_t* Y, uint32_t* c, uint32_t n_begin,
@@ -646,15 +763,10 @@ void launch_crt_pipe(const DevPoint& d, const CrtConsts& cc, const uint32_t* Y, 
     // y: K rows of N words, boxes of 32 primes x 128 coefficients.
     const CUtensorMap tm = make_tmap_u32(Y, static_cast<uint64_t>(d.K), d.N, d.N, kChunk, kCrtTile, TmaSwizzle::kNone);
     const size_t smem = lay.bytes();
-    cudaError_t e = cudaSuccess;
-    switch (d.L) {
-        case 64: e = launch_pdl(k_crt_pipe<64>, dim3(grid), dim3(kThreads), smem, st, d, cc, tm, c, n_begin, n_end, lay); break;
-        case 55: e = launch_pdl(k_crt_pipe<55>, dim3(grid), dim3(kThreads), smem, st, d, cc, tm, c, n_begin, n_end, lay); break;
-        case 28: e = launch_pdl(k_crt_pipe<28>, dim3(grid), dim3(kThreads), smem, st, d, cc, tm, c, n_begin, n_end, lay); break;
-        case 8: e = launch_pdl(k_crt_pipe<8>, dim3(grid), dim3(kThreads), smem, st, d, cc, tm, c, n_begin, n_end, lay); break;
-        default: e = launch_pdl(k_crt_pipe<0>, dim3(grid), dim3(kThreads), smem, st, d, cc, tm, c, n_begin, n_end, lay); break;
-    }
-    check(e, "crt launch");
+    const bool even = (d.L & 3) == 0 && (reinterpret_cast<uintptr_t>(c) & 15) == 0;
+    check(launch_pdl(even ? k_crt_pipe<true> : k_crt_pipe<false>, dim3(grid), dim3(kThreads), smem, st, d, cc, tm, c,
+                     n_begin, n_end, lay),
+          "crt launch");
 }
 
 }  // namespace fpm
