@@ -7,11 +7,10 @@
 //
 // Organisation on the B200: one CTA per SM works on one operand (a pair launch
 // splits the CTAs between a and b) and walks its 128-coefficient tiles:
-//   * warp 0 loads the operand's whole constant image once (chunks of 64
-//     primes x 4 bytes x 4L bytes, the last one packed: at most 160 KB,
-//     resident in shared memory) and then, one thread, issues the MMAs at the
-//     widest shape (N = 256 columns per chunk): D goes to one of two
-//     256-column TMEM buffers;
+//   * warp 0 loads the operand's whole constant image once (equal chunks of at
+//     most 64 primes x 4 bytes x 4L bytes: at most 160 KB, resident in shared
+//     memory) and then, one thread, issues the MMAs, one chunk at a time: D
+//     goes to one of two 256-column TMEM buffers;
 //   * warps 1-4 copy each tile's limbs into a ring of two slots in the MMA's
 //     128-byte-swizzled K-major layout (the layout the tensor cores read at
 //     full rate) with asynchronous copies (cp.async) whose completion the
@@ -21,9 +20,19 @@
 //     the eight lanes of each shared-store phase hit eight different bank
 //     groups;
 //   * warps 5-20, four per TMEM lane quadrant, one coefficient per thread,
-//     each take 16 of a chunk's 64 primes: read D, fold the 49-bit sums mod
+//     each take a quarter of a chunk's primes: read D, fold the 49-bit sums mod
 //     p_j and store the residues (a warp writes 32 consecutive words per
 //     prime).
+// The fold warps' instructions bound it (issue 54% active, tensor pipe 39%,
+// 106 MB in 25.3 us at K = 139, L = 64).  So every fold warp gets the same
+// share of every chunk (K = 139 is 3 chunks of 48 with 12 primes a warp; as 64 +
+// 64 + 11, 16 a warp, the last chunk took as long as a full one), warps whose
+// rows and primes all exist store without a test per prime, and a store's
+// address is one 32-bit add.  Pair launch, before -> after: K = 139 at
+// N = 65536 33.4 -> 25.3 us, K = 71 at N = 2^18 68.0 -> 47.6, K = 36 at
+// N = 2^17 21.7 -> 17.3, K = 60 at N = 32768 9.0 -> 8.2.  The fold constants
+// stay in the parameter bank: from shared memory, which the MMAs load heavily,
+// they took K = 60 from 8.2 to 9.1 us (and K = 139 from 25.3 to 24.4).
 // The fold constants come from kernel parameters.  Every wait is bounded
 // (DevPoint::wait_ns); a timeout raises an abort flag that every role checks,
 // and the error word gets bit 0.
@@ -42,17 +51,17 @@ constexpr int kLoaders = 128;
 constexpr int kEpiWarp0 = 5;                       // warps 5-20
 constexpr int kEpi = 512;
 constexpr uint32_t kRows = 128;
-constexpr uint32_t kCols = 256;                    // GEMM columns per full chunk (64 primes)
+constexpr uint32_t kBufCols = 256;                 // TMEM columns of one of the two buffers
 
 // Operand tiles and the constant image in the 128-byte-swizzle layout
-// (sw128_offset): a tile is 128 rows, a constant chunk 256 columns (the last
-// nlast), each with kb K bytes.
+// (sw128_offset): a tile is 128 rows, a constant chunk `cols` columns, each
+// with kb K bytes.
 __host__ __device__ inline uint32_t a_bytes(uint32_t kb) { return static_cast<uint32_t>(sw128_bytes(kRows, kb)); }
-__host__ __device__ inline size_t b_bytes(uint32_t kb, int nch, uint32_t nlast) {
-    return (static_cast<size_t>(nch) - 1) * sw128_bytes(kCols, kb) + sw128_bytes(nlast, kb);
+__host__ __device__ inline size_t b_bytes(uint32_t kb, int nch, uint32_t cols) {
+    return static_cast<size_t>(nch) * sw128_bytes(cols, kb);
 }
-__host__ inline size_t smem_bytes(uint32_t kb, int nch, uint32_t nlast) {
-    return b_bytes(kb, nch, nlast) + 2 * a_bytes(kb) + 128;
+__host__ inline size_t smem_bytes(uint32_t kb, int nch, uint32_t cols) {
+    return b_bytes(kb, nch, cols) + 2 * a_bytes(kb) + 128;
 }
 
 struct Smem {
@@ -67,10 +76,10 @@ struct Smem {
     volatile uint32_t* abort;
 };
 
-__device__ inline Smem carve(uint8_t* base, uint32_t kb, int nch, uint32_t nlast) {
+__device__ inline Smem carve(uint8_t* base, uint32_t kb, int nch, uint32_t cols) {
     Smem s;
     s.b = base;
-    s.a = base + b_bytes(kb, nch, nlast);
+    s.a = base + b_bytes(kb, nch, cols);
     uint64_t* bars = reinterpret_cast<uint64_t*>(s.a + 2 * a_bytes(kb));
     s.b_full = bars;
     s.a_full = bars + 1;
@@ -105,18 +114,25 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Waits for this thread's two 32-column TMEM loads; naming the registers
-// keeps every read of them below the wait.
-#define FPM_R16(x, o) "+r"(x[o + 0]), "+r"(x[o + 1]), "+r"(x[o + 2]), "+r"(x[o + 3]), "+r"(x[o + 4]), \
-    "+r"(x[o + 5]), "+r"(x[o + 6]), "+r"(x[o + 7]), "+r"(x[o + 8]), "+r"(x[o + 9]), "+r"(x[o + 10]), \
-    "+r"(x[o + 11]), "+r"(x[o + 12]), "+r"(x[o + 13]), "+r"(x[o + 14]), "+r"(x[o + 15])
-__device__ __forceinline__ void tmem_wait2(uint32_t (&r)[2][32]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;" : FPM_R16(r[0], 0)::"memory");
-    asm volatile("" : FPM_R16(r[0], 16)::"memory");
-    asm volatile("" : FPM_R16(r[1], 0)::"memory");
-    asm volatile("" : FPM_R16(r[1], 16)::"memory");
+// Loads NC consecutive columns (a multiple of 8, at most 64) of this thread's
+// TMEM lane and waits for them; naming the registers keeps every read of them
+// below the wait.
+template <int NC>
+__device__ __forceinline__ void tmem_read(uint32_t taddr, uint32_t (&r)[NC]) {
+    static_assert(NC % 8 == 0 && NC <= 64, "columns in eights");
+    int at = 0;
+#pragma unroll
+    for (; at + 32 <= NC; at += 32) tc::tmem_ld32(taddr + at, *reinterpret_cast<uint32_t(*)[32]>(r + at));
+    if constexpr (NC % 32 >= 16) {
+        tc::tmem_ld16(taddr + NC / 32 * 32, *reinterpret_cast<uint32_t(*)[16]>(r + NC / 32 * 32));
+    }
+    if constexpr (NC % 16 == 8) tc::tmem_ld8(taddr + NC - 8, r + NC - 8);
+    tc::tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < NC; i += 8)
+        asm volatile("" : "+r"(r[i]), "+r"(r[i + 1]), "+r"(r[i + 2]), "+r"(r[i + 3]), "+r"(r[i + 4]), "+r"(r[i + 5]),
+                          "+r"(r[i + 6]), "+r"(r[i + 7])::"memory");
 }
-#undef FPM_R16
 
 // A GEMM sum D is below 4L 255^2 <= 256 * 65025 (L <= 64), so both halves of
 // sum_s D_s 2^(8s), A = D_0 + 2^8 D_1 and B = D_2 + 2^8 D_3, are below
@@ -138,7 +154,8 @@ __device__ __forceinline__ uint32_t fold_halves(uint32_t A, uint32_t B, uint4 f)
 }
 
 // CTAs [0, split) take operand 0 (la -> ra), [split, gridDim.x) operand 1.
-template <bool LAZY>
+// P: primes per fold warp and chunk.
+template <int P, bool LAZY>
 __global__ void __launch_bounds__(kThreads, 1)
     k_decompose_pipe(DevPoint d, const __grid_constant__ DecConsts fc, const uint32_t* __restrict__ la,
                      const uint32_t* __restrict__ lb, uint32_t* __restrict__ ra, uint32_t* __restrict__ rb,
@@ -153,9 +170,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     const uint32_t kb = d.dec_kb;
     const int nch = static_cast<int>(fc.chunks);
-    const uint32_t nlast = fc.last_cols;
-    const Smem sm = carve(smem_raw, kb, nch, nlast);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr uint32_t cols = 16 * P;
+    const Smem sm = carve(smem_raw, kb, nch, cols);
+    // (The shuffle tells the compiler that the warp index is uniform.)
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int L = d.L, K = d.K;
     const bool second = blockIdx.x >= split;
     const int operand = operand0 + (second ? 1 : 0);
@@ -164,7 +182,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint8_t* img = fc.img[operand];
     const uint32_t g0 = second ? split : 0, gs = second ? gridDim.x - split : split;
     const uint32_t tiles = (n_end - n_begin + kRows - 1) / kRows;
-    const uint32_t chunk_bytes = static_cast<uint32_t>(sw128_bytes(kCols, kb));
+    const uint32_t chunk_bytes = static_cast<uint32_t>(sw128_bytes(cols, kb));
     const uint64_t lim = d.wait_ns;
 
     if (threadIdx.x == 0) {
@@ -183,13 +201,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         // preceding kernel's tail.
         // (Test hook: with kFaultDecompose the image is never requested, so the
         // MMA issuer's wait for it runs out.)
-        const uint32_t total = static_cast<uint32_t>(b_bytes(kb, nch, nlast));
+        const uint32_t total = static_cast<uint32_t>(b_bytes(kb, nch, cols));
         if (!(d.fault & kFaultDecompose)) {
             tc::mbar_arrive_expect_tx(sm.b_full, total);
-            for (uint32_t off = 0; off < total; off += chunk_bytes) {
-                const uint32_t n = total - off < chunk_bytes ? total - off : chunk_bytes;
-                tc::bulk_g2s(sm.b + off, img + off, n, sm.b_full);
-            }
+            for (uint32_t off = 0; off < total; off += chunk_bytes)
+                tc::bulk_g2s(sm.b + off, img + off, chunk_bytes, sm.b_full);
         }
     }
     if (warp == 0) tc::tmem_alloc(sm.tmem_base, 512);
@@ -202,7 +218,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (warp == 0) {
         // ---- MMA issuer ----
         if (lane == 0) {
-            const uint32_t idesc_full = tc::idesc_u8(kCols), idesc_last = tc::idesc_u8(nlast);
+            constexpr uint32_t idesc = tc::idesc_u8(cols);
             bool ok = tc::wait_or_abort(sm.b_full, 0, sm.abort, lim);
             uint64_t* last_bar = nullptr;   // the barrier of the latest commit
             uint32_t last_par = 0;
@@ -221,14 +237,12 @@ __global__ void __launch_bounds__(kThreads, 1)
                         if (!ok) break;
                     }
                     tc::tc_fence_after();
-                    const bool lastc = c == nch - 1;
-                    const uint32_t cols = lastc ? nlast : kCols;
                     const uint32_t b0 = tc::smem_addr(sm.b + c * chunk_bytes);
                     for (uint32_t kk = 0; kk < kb / 32; ++kk) {
                         const uint32_t half = kk >> 2, step = (kk & 3) * 32;
                         const uint64_t ad = tc::smem_desc_sw128(a0 + half * kRows * 128 + step);
                         const uint64_t bd = tc::smem_desc_sw128(b0 + half * cols * 128 + step);
-                        tc::mma_u8(tmem + buf * kCols, ad, bd, lastc ? idesc_last : idesc_full, kk > 0);
+                        tc::mma_u8(tmem + buf * kBufCols, ad, bd, idesc, kk > 0);
                     }
                     tc::mma_commit(&sm.d_full[buf]);
                     last_bar = &sm.d_full[buf];
@@ -300,15 +314,16 @@ __global__ void __launch_bounds__(kThreads, 1)
         // Whatever is still in flight lands before the CTA may exit.
         cp_async_wait<0>();
     } else {
-        // ---- epilogue: thread = one coefficient, 16 primes of each chunk ----
+        // ---- epilogue: thread = one coefficient, P primes of each chunk ----
         const int ew = warp - kEpiWarp0;
         const uint32_t qd = warp & 3, piece = ew >> 2;
         const uint32_t m = qd * 32 + lane;
-        const uint32_t tq = tmem + ((qd * 32) << 16) + piece * 64;
+        const uint32_t tq = tmem + ((qd * 32) << 16) + piece * (4 * P);
         uint32_t g = 0;
         for (uint32_t t = blockIdx.x - g0; t < tiles; t += gs) {
             const uint32_t n0 = n_begin + t * kRows;
             const bool live = m < min(kRows, n_end - n0);
+            const bool whole = n0 + qd * 32 + 32 <= n_end;   // every row of the warp is live
             bool ok = true;
             for (int c = 0; c < nch; ++c, ++g) {
                 const int buf = g & 1;
@@ -316,32 +331,38 @@ __global__ void __launch_bounds__(kThreads, 1)
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc::tc_fence_after();
-                const int j0 = c * 64 + static_cast<int>(piece) * 16;
-                uint32_t r[2][32];
-                tc::tmem_ld32(tq + buf * kCols, r[0]);
-                tc::tmem_ld32(tq + buf * kCols + 32, r[1]);
-                tmem_wait2(r);
-                // The 32 half-sums are formed before the buffer is released:
+                const int j0 = c * (4 * P) + static_cast<int>(piece) * P;
+                uint32_t r[4 * P];
+                tmem_read<4 * P>(tq + buf * kBufCols, r);
+                // The 2 P half-sums are formed before the buffer is released:
                 // half as many values stay live through the folds.
-                uint32_t hs[16][2];
+                uint32_t hs[P][2];
 #pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    const uint32_t* rr = r[k >> 3] + 4 * (k & 7);
+                for (int k = 0; k < P; ++k) {
+                    const uint32_t* rr = r + 4 * k;
                     hs[k][0] = rr[0] + (rr[1] << 8);
                     hs[k][1] = rr[2] + (rr[3] << 8);
                 }
                 tc::tc_fence_before();
                 tc::mbar_arrive(&sm.d_empty[buf]);
-                if (j0 < K) {
-                    // One running pointer down the primes' rows (no 64-bit
-                    // product per store).
-                    uint32_t* out = res + static_cast<size_t>(j0) * d.N + n0 + m;
-                    const size_t stride = d.N;
+                // Byte offsets into the residues fit 32 bits (K N words below
+                // 2^30), one add a prime.
+                uint32_t at = (static_cast<uint32_t>(j0) * d.N + n0 + m) * 4u;
+                const uint32_t stride = d.N * 4u;
+                uint8_t* out = reinterpret_cast<uint8_t*>(res);
+                if (whole && j0 + P <= K) {
 #pragma unroll
-                    for (int k = 0; k < 16; ++k) {
-                        const int j = j0 + k;
-                        if (live && j < K) *out = fold_halves<LAZY>(hs[k][0], hs[k][1], fc.fold[j]);
-                        out += stride;
+                    for (int k = 0; k < P; ++k) {
+                        *reinterpret_cast<uint32_t*>(out + at) = fold_halves<LAZY>(hs[k][0], hs[k][1], fc.fold[j0 + k]);
+                        at += stride;
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < P; ++k) {
+                        if (live && j0 + k < K)
+                            *reinterpret_cast<uint32_t*>(out + at) =
+                                fold_halves<LAZY>(hs[k][0], hs[k][1], fc.fold[j0 + k]);
+                        at += stride;
                     }
                 }
             }
@@ -366,23 +387,45 @@ DecConsts make_dec_consts(const HostPlan& pl, const uint8_t* img_a, const uint8_
     dc.img[0] = img_a;
     dc.img[1] = img_b;
     dc.chunks = pl.dec_wchunks;
-    dc.last_cols = pl.dec_wlast;
+    dc.piece = pl.dec_wpiece;
     // The four-step transforms start with lazy butterflies; the one-block
     // transform (N <= 1024) and the full-reduction window want canonical input.
     dc.lazy_out = pl.lazy && pl.g.logN > kSmallLogN ? 1u : 0u;
     return dc;
 }
 
+namespace {
+
+using DecKernel = void (*)(DevPoint, const DecConsts, const uint32_t*, const uint32_t*, uint32_t*, uint32_t*, int,
+                           uint32_t, uint32_t, uint32_t);
+
+template <bool LAZY>
+DecKernel dec_kernel(uint32_t piece) {
+    switch (piece) {
+        case 2: return k_decompose_pipe<2, LAZY>;
+        case 4: return k_decompose_pipe<4, LAZY>;
+        case 6: return k_decompose_pipe<6, LAZY>;
+        case 8: return k_decompose_pipe<8, LAZY>;
+        case 10: return k_decompose_pipe<10, LAZY>;
+        case 12: return k_decompose_pipe<12, LAZY>;
+        case 14: return k_decompose_pipe<14, LAZY>;
+        case 16: return k_decompose_pipe<16, LAZY>;
+        default: throw std::runtime_error("decompose: unsupported chunk size");
+    }
+}
+
+}  // namespace
+
 bool decompose_pipe_supported(const HostPlan& pl) {
-    return pl.K <= kMaxK && pl.dec_wchunks >= 1 && pl.dec_wlast >= 16 && pl.dec_wlast <= 256 &&
-           smem_bytes(pl.dec_kb, static_cast<int>(pl.dec_wchunks), pl.dec_wlast) <= 227 * 1024;
+    return pl.K <= kMaxK && pl.dec_wchunks >= 1 && pl.dec_wpiece >= 2 && pl.dec_wpiece <= 16 &&
+           smem_bytes(pl.dec_kb, static_cast<int>(pl.dec_wchunks), 16 * pl.dec_wpiece) <= 227 * 1024;
 }
 
 void decompose_pipe_init_attributes() {
-    check(cudaFuncSetAttribute(k_decompose_pipe<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024),
-          "decompose_pipe smem");
-    check(cudaFuncSetAttribute(k_decompose_pipe<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024),
-          "decompose_pipe smem");
+    for (uint32_t piece = 2; piece <= 16; piece += 2)
+        for (DecKernel k : {dec_kernel<false>(piece), dec_kernel<true>(piece)})
+            check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024),
+                  "decompose_pipe smem");
 }
 
 void launch_decompose_pipe(const DevPoint& d, const DecConsts& dc, const uint32_t* a, const uint32_t* b,
@@ -397,8 +440,8 @@ void launch_decompose_pipe(const DevPoint& d, const DecConsts& dc, const uint32_
     if (per > tiles) per = tiles;
     const uint32_t grid = per * operands;
     const uint32_t split = operands == 2 ? per : grid;
-    check(launch_pdl(dc.lazy_out ? k_decompose_pipe<true> : k_decompose_pipe<false>, dim3(grid), dim3(kThreads),
-                     smem_bytes(d.dec_kb, static_cast<int>(dc.chunks), dc.last_cols), st, d, dc, a,
+    check(launch_pdl(dc.lazy_out ? dec_kernel<true>(dc.piece) : dec_kernel<false>(dc.piece), dim3(grid),
+                     dim3(kThreads), smem_bytes(d.dec_kb, static_cast<int>(dc.chunks), 16 * dc.piece), st, d, dc, a,
                      b ? b : a, A, B ? B : A, operand0, n_begin, n_end, split),
           "decompose launch");
 }

@@ -105,8 +105,8 @@ void launch_crt_pipe(const DevPoint& d, const CrtConsts& cc, const uint32_t* Y, 
 struct DecConsts {
     uint4 fold[kMaxK];          // {p, 2^16 mod p, its Shoup companion, floor(2^32 / p)}
     const uint8_t* img[2];      // device copies of the plan's wide images, operands a and b
-    uint32_t chunks;            // chunks of 64 primes
-    uint32_t last_cols;         // GEMM columns of the last chunk
+    uint32_t chunks;            // chunks of 4 piece primes (16 piece GEMM columns)
+    uint32_t piece;             // primes per fold warp and chunk: 2, 4 .. 16
     uint32_t lazy_out;          // 1: residues below 4p (congruent), for lazy first butterflies
 };
 DecConsts make_dec_consts(const HostPlan& pl, const uint8_t* img_a, const uint8_t* img_b);

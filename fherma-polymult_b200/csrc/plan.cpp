@@ -274,12 +274,16 @@ HostPlan make_plan_basis(uint32_t N, uint32_t W, int L, int qbits, int pmax_log2
     pl.dec_img_a.assign(dchunk * pl.dec_chunks, 0);
     pl.dec_img_b.assign(dchunk * pl.dec_chunks, 0);
     pl.dec_fold.resize(K);
-    // Wide images: chunks of 64 primes (256 GEMM columns, the MMA's widest N);
-    // the last chunk packed to its own width, a multiple of 16 columns.
+    // Wide images: the fewest chunks of at most 64 primes (256 GEMM columns,
+    // the MMA's widest N), all of one size: the pipeline's four fold warps per
+    // lane quadrant take a quarter of a chunk each, and a chunk costs them the
+    // same however few of its columns are used.  A quarter is an even number
+    // of primes (TMEM is read two primes at a time).
     pl.dec_wchunks = static_cast<uint32_t>((K + 63) / 64);
-    pl.dec_wlast = (4 * static_cast<uint32_t>(K - 64 * (static_cast<int>(pl.dec_wchunks) - 1)) + 15) / 16 * 16;
-    const size_t wchunk = sw128_bytes(256, pl.dec_kb);   // 128-byte-swizzle layout (sw128_offset)
-    pl.dec_wimg_a.assign(wchunk * (pl.dec_wchunks - 1) + sw128_bytes(pl.dec_wlast, pl.dec_kb), 0);
+    pl.dec_wpiece = (static_cast<uint32_t>(K) + 8 * pl.dec_wchunks - 1) / (8 * pl.dec_wchunks) * 2;
+    const uint32_t wprimes = 4 * pl.dec_wpiece, wcols = 4 * wprimes;
+    const size_t wchunk = sw128_bytes(wcols, pl.dec_kb);   // 128-byte-swizzle layout (sw128_offset)
+    pl.dec_wimg_a.assign(wchunk * pl.dec_wchunks, 0);
     pl.dec_wimg_b.assign(pl.dec_wimg_a.size(), 0);
     for (int j = 0; j < K; ++j) {
         const uint32_t p = pl.primes[j];
@@ -295,8 +299,7 @@ HostPlan make_plan_basis(uint32_t N, uint32_t W, int L, int qbits, int pmax_log2
                 const size_t at = chunk + (k / 16) * (128 * 16) + col * 16 + (k % 16);
                 pl.dec_img_a[at] = static_cast<uint8_t>(ca >> (8 * s));
                 pl.dec_img_b[at] = static_cast<uint8_t>(cb >> (8 * s));
-                const uint32_t wc = static_cast<uint32_t>(j / 64), wcol = 4 * (j % 64) + s;
-                const uint32_t wcols = wc + 1 < pl.dec_wchunks ? 256 : pl.dec_wlast;
+                const uint32_t wc = static_cast<uint32_t>(j) / wprimes, wcol = 4 * (j % wprimes) + s;
                 const size_t wat = wc * wchunk + sw128_offset(wcol, k, wcols);
                 pl.dec_wimg_a[wat] = static_cast<uint8_t>(ca >> (8 * s));
                 pl.dec_wimg_b[wat] = static_cast<uint8_t>(cb >> (8 * s));

@@ -85,11 +85,11 @@ struct HostPlan {
     uint32_t dec_kb = 0;                     // GEMM K in bytes: 4L rounded up to 32
     uint32_t dec_chunks = 0;                 // ceil(K / 32)
     std::vector<uint8_t> dec_img_a, dec_img_b;
-    // The same constants in chunks of 64 primes (256 columns) for the
-    // pipelined decompose, in the UMMA K-major 128-byte-swizzle layout
-    // (sw128_offset, one block per 128 K bytes); the last chunk has
-    // dec_wlast columns.
-    uint32_t dec_wchunks = 0, dec_wlast = 0;
+    // The same constants for the pipelined decompose in dec_wchunks equal
+    // chunks of 4 dec_wpiece primes (16 dec_wpiece columns, the last chunk
+    // padded with zero columns), in the UMMA K-major 128-byte-swizzle layout
+    // (sw128_offset, one block per 128 K bytes).
+    uint32_t dec_wchunks = 0, dec_wpiece = 0;
     std::vector<uint8_t> dec_wimg_a, dec_wimg_b;
     std::vector<uint4> dec_fold;             // K: {p, 2^16 mod p, its Shoup companion, floor(2^32 / p)}
 
