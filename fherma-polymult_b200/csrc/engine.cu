@@ -137,6 +137,11 @@ private:
             build_row_tables(d, tw, nullptr);
             check(cudaDeviceSynchronize(), "row tables");
             d.row_tw = tw;
+        } else if (pl.g.logN >= kWholeMinLogN) {
+            uint2* tw = mem.alloc<uint2>(static_cast<size_t>(pl.K) * pl.N);
+            build_whole_tables(d, tw, nullptr);
+            check(cudaDeviceSynchronize(), "transform tables");
+            d.row_tw = tw;
         }
         for (auto* v : {&pl.dec_a, &pl.dec_b, &pl.col_f, &pl.col_i, &pl.row_u_f, &pl.row_q_f, &pl.full_f, &pl.full_i})
             drop(*v);

@@ -59,6 +59,15 @@ void launch_ntt(const DevPoint& d, uint32_t* A, uint32_t* B, int mode, cudaStrea
 // point's generators row_u_f and row_q_f; once per context.
 void build_row_tables(const DevPoint& d, uint2* out, cudaStream_t st);
 
+// The whole chain in one launch (ntt_fused.cu): N = 2^8 .. 2^11 in a block per
+// prime (products and forward transforms), N = 2^12 .. 2^15 in a cluster per
+// prime (products whose clusters are all resident at once).  N = 2^8 .. 2^10 read tables of their own, K x N pairs from
+// build_whole_tables (DevPoint::row_tw).
+bool ntt_fused_ok(const DevPoint& d, int mode, int sms);
+void launch_ntt_fused(const DevPoint& d, uint32_t* A, uint32_t* B, int mode, cudaStream_t st);
+void build_whole_tables(const DevPoint& d, uint2* out, cudaStream_t st);
+void ntt_fused_init_attributes();
+
 // The same on the tensor cores.
 void launch_decompose_tc(const DevPoint& d, const uint32_t* limbs, uint32_t* res, int operand, uint32_t n_begin,
                          uint32_t n_end, cudaStream_t st);

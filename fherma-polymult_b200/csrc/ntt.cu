@@ -25,6 +25,7 @@
 #include "group.cuh"
 #include "kernels.h"
 #include "ntt_engine.cuh"
+#include "ntt_passes.cuh"
 #include "pdl.cuh"
 #include "tc.cuh"
 #include "tmap.h"
@@ -32,75 +33,10 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
-#include <type_traits>
 
 namespace fpm {
 
 namespace {
-
-template <int NSUB, int XS, class SWZ, int RB>
-using RP = Rounds<NSUB, XS, SWZ, RB>;
-
-// Column-pass shared layout for RB register bits.
-template <int RB>
-using SwzC = std::conditional_t<RB == 3, SwzCol, SwzRow>;
-
-// The threads that own one tile: the whole block, or one 128-thread half of a
-// 256-thread block (the grouped row pass of mixed geometries runs two
-// 128-thread tiles per block).
-struct BlockTeam {
-    static __device__ __forceinline__ uint32_t tid() { return threadIdx.x; }
-    static __device__ __forceinline__ void sync() { __syncthreads(); }
-};
-struct HalfTeam {
-    static __device__ __forceinline__ uint32_t tid() { return threadIdx.x & 127u; }
-    static __device__ __forceinline__ void sync() {
-        asm volatile("bar.sync %0, 128;" ::"r"(1u + (threadIdx.x >> 7)) : "memory");
-    }
-};
-
-// Round R through shared memory on NV tiles.
-template <int NSUB, int XS, class SWZ, int RB, int R, bool LAZY, int NV, class TEAM = BlockTeam, class TW>
-__device__ __forceinline__ void fwd_step(uint32_t* const (&tiles)[NV], const TW& tw, uint32_t p) {
-    const uint32_t base = round_base<NSUB, XS, SWZ, RB, R>(TEAM::tid());
-    uint32_t v[NV][1 << RB];
-#pragma unroll
-    for (int o = 0; o < NV; ++o) load_round<NSUB, XS, SWZ, RB, R>(tiles[o], v[o], base);
-    fwd_round<NSUB, XS, SWZ, RB, R, LAZY, NV>(v, base, tw, p);
-#pragma unroll
-    for (int o = 0; o < NV; ++o) store_round<NSUB, XS, SWZ, RB, R>(tiles[o], v[o], base);
-    TEAM::sync();
-}
-
-template <int NSUB, int XS, class SWZ, int RB, int R, int REND, bool LAZY, int NV, class TEAM = BlockTeam,
-          class TW>
-__device__ __forceinline__ void fwd_range(uint32_t* const (&tiles)[NV], const TW& tw, uint32_t p) {
-    if constexpr (R < REND) {
-        fwd_step<NSUB, XS, SWZ, RB, R, LAZY, NV, TEAM>(tiles, tw, p);
-        fwd_range<NSUB, XS, SWZ, RB, R + 1, REND, LAZY, NV, TEAM>(tiles, tw, p);
-    }
-}
-
-// Inverse rounds R, R - 1, ..., RLO through shared memory.
-template <int NSUB, int XS, class SWZ, int RB, int R, int RLO, bool LAZY, bool NEG, class TEAM = BlockTeam,
-          class TW>
-__device__ __forceinline__ void inv_range(uint32_t* tile, const TW& tw, uint32_t p) {
-    if constexpr (R >= RLO) {
-        const uint32_t base = round_base<NSUB, XS, SWZ, RB, R>(TEAM::tid());
-        uint32_t v[1 << RB];
-        load_round<NSUB, XS, SWZ, RB, R>(tile, v, base);
-        inv_round<NSUB, XS, SWZ, RB, R, LAZY, NEG>(v, base, tw, p);
-        store_round<NSUB, XS, SWZ, RB, R>(tile, v, base);
-        TEAM::sync();
-        inv_range<NSUB, XS, SWZ, RB, R - 1, RLO, LAZY, NEG, TEAM>(tile, tw, p);
-    }
-}
-
-// Canonical residue from a lazy one (< 4p).
-__device__ __forceinline__ uint32_t canon4(uint32_t x, uint32_t p) {
-    x = umin32(x, x - 2 * p);
-    return umin32(x, x - p);
-}
 
 // ---------------------------------------------------------------------------
 // Column pass: a block owns C = 2^XS adjacent columns c0 .. c0 + C - 1 of one
@@ -108,40 +44,6 @@ __device__ __forceinline__ uint32_t canon4(uint32_t x, uint32_t p) {
 // sub-transform, column c = sub-transform).  Element (u, c) is X[u S + c0 + c].
 // S = 2^LOGS is a template parameter too, so a thread's strided global
 // accesses are one base address plus immediates.
-
-template <int LOGR, int LOGS>
-__device__ __forceinline__ uint32_t col_offset(uint32_t i, uint32_t c0) {
-    constexpr int XS = 11 - LOGR;
-    return ((i >> XS) << LOGS) + c0 + (i & ((1u << XS) - 1u));
-}
-
-template <int LOGR, int LOGS, int RB, int R, int NV>
-__device__ __forceinline__ void col_global_load(const uint32_t* const (&X)[NV], uint32_t (&v)[NV][1 << RB],
-                                                uint32_t base, uint32_t c0) {
-    constexpr int XS = 11 - LOGR, sh = RP<LOGR, XS, SwzC<RB>, RB>::lo(R);
-    constexpr uint32_t step = (1u << LOGS) << sh;
-    const uint32_t at = col_offset<LOGR, LOGS>(base, c0);
-#pragma unroll
-    for (int o = 0; o < NV; ++o) {
-        const uint32_t* x = X[o] + at;
-#pragma unroll
-        for (int k = 0; k < (1 << RB); ++k) v[o][k] = x[k * step];
-    }
-}
-
-template <int LOGR, int LOGS, int RB, int R, int NV>
-__device__ __forceinline__ void col_global_store(uint32_t* const (&X)[NV], const uint32_t (&v)[NV][1 << RB],
-                                                 uint32_t base, uint32_t c0) {
-    constexpr int XS = 11 - LOGR, sh = RP<LOGR, XS, SwzC<RB>, RB>::lo(R);
-    constexpr uint32_t step = (1u << LOGS) << sh;
-    const uint32_t at = col_offset<LOGR, LOGS>(base, c0);
-#pragma unroll
-    for (int o = 0; o < NV; ++o) {
-        uint32_t* x = X[o] + at;
-#pragma unroll
-        for (int k = 0; k < (1 << RB); ++k) x[k * step] = v[o][k];
-    }
-}
 
 template <int LOGR, int LOGS, bool LAZY>
 __device__ __forceinline__ void col_fwd_body(const DevPoint& d, uint32_t* A, uint32_t* B, int j, uint32_t bx) {
@@ -412,26 +314,6 @@ __global__ void __launch_bounds__(256, 8) k_ntt_col_inv_tma(DevPoint d, const __
 // per context (K x R x S pairs); a row block copies its rows' tables into
 // shared memory asynchronously.
 
-template <int LOGS>
-struct RowGeom {
-    static constexpr uint32_t S = 1u << LOGS;
-    static constexpr uint32_t G = 2048u >> LOGS;
-    static constexpr uint32_t kSlots = G >= 2 ? G : 2;
-    static constexpr uint32_t kStride = S + 4;                 // entries; pads rows across banks
-    static constexpr uint32_t kFlip = G >= 2 ? G / 2 : 1;
-    static constexpr uint32_t kPairsPerBlock = G >= 2 ? G / 2 : 1;
-};
-
-template <int LOGS>
-__device__ __forceinline__ uint32_t row_of_slot(uint32_t slot, uint32_t u0, uint32_t R) {
-    using RG = RowGeom<LOGS>;
-    if constexpr (RG::G >= 2) {
-        return slot < RG::G / 2 ? u0 + slot : R - 1 - u0 - (slot - RG::G / 2);
-    } else {
-        return slot == 0 ? u0 : R - 1 - u0;
-    }
-}
-
 // Copies the block's row tables (slot s holds row row_of_slot(s)) from the
 // prebuilt K x R x S array into shared memory with bulk asynchronous copies
 // (one per row table, S Shoup pairs, issued by the lanes of warp 0), counted
@@ -558,15 +440,7 @@ __device__ __forceinline__ void row_body(const DevPoint& d, uint32_t* A, uint32_
             return;
         }
 #pragma unroll
-        for (int k = 0; k < E; ++k) {
-            uint32_t x = v[0][k], y = v[1][k];
-            if constexpr (LAZY) {
-                // below 2p each, so the Montgomery product stays below 2p
-                x = umin32(x, x - 2 * p);
-                y = umin32(y, y - 2 * p);
-            }
-            v[0][k] = mont_mul(x, y, p, pc.pneg);
-        }
+        for (int k = 0; k < E; ++k) v[0][k] = pointwise<LAZY>(v[0][k], v[1][k], pc);
         inv_round<LOGS, 0, SwzRow, RB, last, LAZY, true>(v[0], base, iw, p);
         store_round<LOGS, 0, SwzRow, RB, last>(ta, v[0], base);
         TEAM::sync();
@@ -795,8 +669,8 @@ __global__ void __launch_bounds__(256, 3) k_ntt_row_mixed(const __grid_constant_
 }
 
 // ---------------------------------------------------------------------------
-// N <= 1024: one block per prime holds both operands; one butterfly per
-// thread per stage, full twiddle tables from global memory, full reduction.
+// N < 256: one block per prime holds both operands; one butterfly per thread
+// per stage, full twiddle tables from global memory, full reduction.
 
 __global__ void __launch_bounds__(kNttThreads) k_ntt_small(DevPoint d, uint32_t* A, uint32_t* B, int mode) {
     extern __shared__ __align__(1024) uint32_t smem[];
@@ -970,8 +844,7 @@ void attrs_all() {
     row_attrs<11, LAZY>();
 }
 
-// SMs of the current device (the persistent column grids take one slot per
-// resident CTA).
+// SMs of the current device.
 int device_sms() {
     static int cached[64] = {};
     int dev = 0;
@@ -1181,6 +1054,7 @@ void build_row_tables(const DevPoint& d, uint2* out, cudaStream_t st) {
 }
 
 void ntt_init_attributes() {
+    ntt_fused_init_attributes();
     attrs_all<true>();
     attrs_all<false>();
     mixed_attrs<true>();
@@ -1193,6 +1067,13 @@ void ntt_init_attributes() {
 // mode kRowForward stops after the forward transforms (A, B bit-reversed,
 // canonical).
 void launch_ntt(const DevPoint& d, uint32_t* A, uint32_t* B, int mode, cudaStream_t st) {
+    // A transform without column passes is its row pass; FPM_COL_PASS asks for
+    // the separate passes where there are any.
+    const int m = d.logR == 0 && mode == kPassRow ? static_cast<int>(kRowProduct) : mode;
+    if (ntt_fused_ok(d, m, device_sms()) && (d.logR == 0 || col_pass_variant() == 0)) {
+        launch_ntt_fused(d, A, B, m, st);
+        return;
+    }
     if (d.logN <= kSmallLogN) {
         if (mode == kRowProduct || mode == kRowForward || mode == kPassRow)
             k_ntt_small<<<d.K, kNttThreads, 2 * d.N * sizeof(uint32_t), st>>>(d, A, B,

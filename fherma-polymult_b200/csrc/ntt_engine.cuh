@@ -1,4 +1,5 @@
-// Register-blocked NTT rounds on a 2048-element shared-memory tile.
+// Register-blocked NTT rounds on a shared-memory tile of 2^BITS elements (2048
+// but for the transforms of N <= 1024, whose tile is the whole polynomial).
 //
 // A tile holds 2048 / 2^NSUB independent sub-transforms of 2^NSUB elements.  The
 // tile index i carries the position x inside a sub-transform in bits
@@ -47,30 +48,37 @@ constexpr int kNttThreads = ntt_threads<3>();
 
 // Row-pass layout: bank bit c of word i is i_c ^ i_{c+5}.  Any window of four
 // contiguous register bits holds at most one of c, c + 5.
-struct SwzRow {
+// (BITS: log2 of the tile's elements.)
+template <int BITS>
+struct SwzRowT {
+    static constexpr int kBits = BITS;
     static constexpr __host__ __device__ uint32_t f(uint32_t i) { return i ^ ((i >> 5) & 31u); }
     static constexpr __host__ __device__ int partner(int c) { return c + 5; }
 };
+using SwzRow = SwzRowT<11>;
 // Column layout for 8-element rounds: the 128-byte TMA swizzle (16-byte chunk
 // index ^= 128-byte line index mod 8); bank bits 0, 1 are i_0, i_1 and bank bit
 // c >= 2 is i_c ^ i_{c+3}.  (A 4-bit register window can hold c and c + 3, so
 // 16-element rounds use SwzRow.)
 struct SwzCol {
+    static constexpr int kBits = 11;
     static constexpr __host__ __device__ uint32_t f(uint32_t i) { return i ^ (((i >> 5) & 7u) << 2); }
     static constexpr __host__ __device__ int partner(int c) { return c >= 2 ? c + 3 : -1; }
 };
 
 struct RoundMap {
     int lane[5];
-    int warp[3];
+    int warp[4];
 };
 
 template <int NSUB, int XS, class SWZ, int RB = 3>
 struct Rounds {
     static_assert(RB == 3 || RB == 4, "8 or 16 elements per thread");
-    static_assert(NSUB >= 6 && NSUB <= 11 && XS + NSUB <= 11, "2^6 .. 2^11-element sub-transforms");
+    static constexpr int kBits = SWZ::kBits;
+    static_assert(NSUB >= 6 && NSUB <= 11 && XS + NSUB <= kBits, "2^6 .. 2^11-element sub-transforms");
     static constexpr int kRegs = 1 << RB;
-    static constexpr int kWarpBits = 6 - RB;
+    static constexpr int kWarpBits = kBits - 5 - RB;
+    static_assert(kWarpBits >= 0, "a warp at least");
     static constexpr int kCount = (NSUB + RB - 1) / RB;
     static constexpr __host__ __device__ int cnt(int r) { return (r < kCount - 1 || NSUB % RB == 0) ? RB : NSUB % RB; }
     static constexpr __host__ __device__ int lo(int r) { return NSUB - RB * r - cnt(r); }
@@ -79,8 +87,8 @@ struct Rounds {
     }
     static constexpr __host__ __device__ RoundMap map(int r) {
         RoundMap m{};
-        bool used[11] = {};
-        for (int b = 0; b < 11; ++b) used[b] = is_reg(r, b);
+        bool used[kBits] = {};
+        for (int b = 0; b < kBits; ++b) used[b] = is_reg(r, b);
         // lane bits: bank bit c itself, else its swizzle partner, else any free bit
         for (int c = 0; c < 5; ++c) {
             int pick = -1;
@@ -88,10 +96,10 @@ struct Rounds {
                 pick = c;
             } else {
                 const int pc = SWZ::partner(c);
-                if (pc >= 0 && pc < 11 && !used[pc]) pick = pc;
+                if (pc >= 0 && pc < kBits && !used[pc]) pick = pc;
             }
             if (pick < 0) {
-                for (int b = 0; b < 11 && pick < 0; ++b)
+                for (int b = 0; b < kBits && pick < 0; ++b)
                     if (!used[b]) pick = b;
             }
             m.lane[c] = pick;
@@ -108,7 +116,7 @@ struct Rounds {
                     m.lane[c + 1] = s;
                 }
         int w = 0;
-        for (int b = 0; b < 11; ++b)
+        for (int b = 0; b < kBits; ++b)
             if (!used[b]) m.warp[w++] = b;
         return m;
     }
@@ -140,6 +148,10 @@ struct Rounds {
 // block cost twice as many entries per thread with 16-element rounds.)
 constexpr __host__ __device__ int col_pass_rb(int log) { return (log + 3) / 4 < (log + 2) / 3 ? 4 : 3; }
 constexpr __host__ __device__ int row_pass_rb(int log) { return col_pass_rb(log); }
+// One-block transforms of N = 2^log: 8 elements, for threads (N / 8 per
+// operand) where a single block is all an SM has; N = 2048 has the row pass's
+// tables, so its register bits.
+constexpr __host__ __device__ int whole_pass_rb(int log) { return log == 11 ? row_pass_rb(11) : 3; }
 
 // Twiddle-table layout of the row pass ("round-major").  Level l of a table
 // (entries [2^l, 2^(l+1)), the stage of distance 2^(NSUB-1-l)) is read in round
@@ -177,7 +189,7 @@ template <int NSUB, int XS, class SWZ, int RB, int R, bool LANE>
 __device__ __forceinline__ uint32_t deposit(uint32_t x) {
     uint32_t b = 0;
 #pragma unroll
-    for (int sh = 0; sh <= 10; ++sh) {
+    for (int sh = 0; sh < SWZ::kBits; ++sh) {
         const uint32_t mask = deposit_mask<NSUB, XS, SWZ, RB, R, LANE>(sh);
         if (mask) b |= (x & mask) << sh;
     }

@@ -1,0 +1,146 @@
+// Device building blocks shared by the transform kernels: rounds through
+// shared memory, a column tile's global accesses, and the rows of a row tile.
+#pragma once
+
+#include "device.cuh"
+#include "ntt_engine.cuh"
+
+#include <type_traits>
+
+namespace fpm {
+
+namespace {
+
+template <int NSUB, int XS, class SWZ, int RB>
+using RP = Rounds<NSUB, XS, SWZ, RB>;
+
+// Column-pass shared layout for RB register bits.
+template <int RB>
+using SwzC = std::conditional_t<RB == 3, SwzCol, SwzRow>;
+
+// The threads that own one tile: the whole block, or one 128-thread half of a
+// 256-thread block (the grouped row pass of mixed geometries runs two
+// 128-thread tiles per block).
+struct BlockTeam {
+    static __device__ __forceinline__ uint32_t tid() { return threadIdx.x; }
+    static __device__ __forceinline__ void sync() { __syncthreads(); }
+};
+struct HalfTeam {
+    static __device__ __forceinline__ uint32_t tid() { return threadIdx.x & 127u; }
+    static __device__ __forceinline__ void sync() {
+        asm volatile("bar.sync %0, 128;" ::"r"(1u + (threadIdx.x >> 7)) : "memory");
+    }
+};
+
+// Round R through shared memory on NV tiles.
+template <int NSUB, int XS, class SWZ, int RB, int R, bool LAZY, int NV, class TEAM = BlockTeam, class TW>
+__device__ __forceinline__ void fwd_step(uint32_t* const (&tiles)[NV], const TW& tw, uint32_t p) {
+    const uint32_t base = round_base<NSUB, XS, SWZ, RB, R>(TEAM::tid());
+    uint32_t v[NV][1 << RB];
+#pragma unroll
+    for (int o = 0; o < NV; ++o) load_round<NSUB, XS, SWZ, RB, R>(tiles[o], v[o], base);
+    fwd_round<NSUB, XS, SWZ, RB, R, LAZY, NV>(v, base, tw, p);
+#pragma unroll
+    for (int o = 0; o < NV; ++o) store_round<NSUB, XS, SWZ, RB, R>(tiles[o], v[o], base);
+    TEAM::sync();
+}
+
+template <int NSUB, int XS, class SWZ, int RB, int R, int REND, bool LAZY, int NV, class TEAM = BlockTeam,
+          class TW>
+__device__ __forceinline__ void fwd_range(uint32_t* const (&tiles)[NV], const TW& tw, uint32_t p) {
+    if constexpr (R < REND) {
+        fwd_step<NSUB, XS, SWZ, RB, R, LAZY, NV, TEAM>(tiles, tw, p);
+        fwd_range<NSUB, XS, SWZ, RB, R + 1, REND, LAZY, NV, TEAM>(tiles, tw, p);
+    }
+}
+
+// Inverse rounds R, R - 1, ..., RLO through shared memory.
+template <int NSUB, int XS, class SWZ, int RB, int R, int RLO, bool LAZY, bool NEG, class TEAM = BlockTeam,
+          class TW>
+__device__ __forceinline__ void inv_range(uint32_t* tile, const TW& tw, uint32_t p) {
+    if constexpr (R >= RLO) {
+        const uint32_t base = round_base<NSUB, XS, SWZ, RB, R>(TEAM::tid());
+        uint32_t v[1 << RB];
+        load_round<NSUB, XS, SWZ, RB, R>(tile, v, base);
+        inv_round<NSUB, XS, SWZ, RB, R, LAZY, NEG>(v, base, tw, p);
+        store_round<NSUB, XS, SWZ, RB, R>(tile, v, base);
+        TEAM::sync();
+        inv_range<NSUB, XS, SWZ, RB, R - 1, RLO, LAZY, NEG, TEAM>(tile, tw, p);
+    }
+}
+
+// Canonical residue from a lazy one (< 4p).
+__device__ __forceinline__ uint32_t canon4(uint32_t x, uint32_t p) {
+    x = umin32(x, x - 2 * p);
+    return umin32(x, x - p);
+}
+
+// The pointwise product of two forward transforms' values (lazy ones below 4p):
+// x y 2^-32 mod p, below 2p (lazy) or canonical.
+template <bool LAZY>
+__device__ __forceinline__ uint32_t pointwise(uint32_t x, uint32_t y, const PrimeConsts& pc) {
+    if constexpr (LAZY) {
+        // below 2p each, so the Montgomery product stays below 2p
+        x = umin32(x, x - 2 * pc.p);
+        y = umin32(y, y - 2 * pc.p);
+    }
+    return mont_mul(x, y, pc.p, pc.pneg);
+}
+
+template <int LOGR, int LOGS>
+__device__ __forceinline__ uint32_t col_offset(uint32_t i, uint32_t c0) {
+    constexpr int XS = 11 - LOGR;
+    return ((i >> XS) << LOGS) + c0 + (i & ((1u << XS) - 1u));
+}
+
+template <int LOGR, int LOGS, int RB, int R, int NV>
+__device__ __forceinline__ void col_global_load(const uint32_t* const (&X)[NV], uint32_t (&v)[NV][1 << RB],
+                                                uint32_t base, uint32_t c0) {
+    constexpr int XS = 11 - LOGR, sh = RP<LOGR, XS, SwzC<RB>, RB>::lo(R);
+    constexpr uint32_t step = (1u << LOGS) << sh;
+    const uint32_t at = col_offset<LOGR, LOGS>(base, c0);
+#pragma unroll
+    for (int o = 0; o < NV; ++o) {
+        const uint32_t* x = X[o] + at;
+#pragma unroll
+        for (int k = 0; k < (1 << RB); ++k) v[o][k] = x[k * step];
+    }
+}
+
+template <int LOGR, int LOGS, int RB, int R, int NV>
+__device__ __forceinline__ void col_global_store(uint32_t* const (&X)[NV], const uint32_t (&v)[NV][1 << RB],
+                                                 uint32_t base, uint32_t c0) {
+    constexpr int XS = 11 - LOGR, sh = RP<LOGR, XS, SwzC<RB>, RB>::lo(R);
+    constexpr uint32_t step = (1u << LOGS) << sh;
+    const uint32_t at = col_offset<LOGR, LOGS>(base, c0);
+#pragma unroll
+    for (int o = 0; o < NV; ++o) {
+        uint32_t* x = X[o] + at;
+#pragma unroll
+        for (int k = 0; k < (1 << RB); ++k) x[k * step] = v[o][k];
+    }
+}
+
+template <int LOGS>
+struct RowGeom {
+    static constexpr uint32_t S = 1u << LOGS;
+    static constexpr uint32_t G = 2048u >> LOGS;
+    static constexpr uint32_t kSlots = G >= 2 ? G : 2;
+    static constexpr uint32_t kStride = S + 4;                 // entries; pads rows across banks
+    static constexpr uint32_t kFlip = G >= 2 ? G / 2 : 1;
+    static constexpr uint32_t kPairsPerBlock = G >= 2 ? G / 2 : 1;
+};
+
+template <int LOGS>
+__device__ __forceinline__ uint32_t row_of_slot(uint32_t slot, uint32_t u0, uint32_t R) {
+    using RG = RowGeom<LOGS>;
+    if constexpr (RG::G >= 2) {
+        return slot < RG::G / 2 ? u0 + slot : R - 1 - u0 - (slot - RG::G / 2);
+    } else {
+        return slot == 0 ? u0 : R - 1 - u0;
+    }
+}
+
+}  // namespace
+
+}  // namespace fpm

@@ -18,8 +18,9 @@ namespace fpm {
 
 // How the length-N transform is cut for the kernels.
 //   logN <= kSmallLogN : one block per prime holds the whole transform
-//                        (k_ntt_small), full twiddle tables.
-//   logN == 11         : one 2048-element tile per prime (row kernel, R = 1).
+//                        (k_ntt_small, from 2^kWholeMinLogN up k_ntt_whole),
+//                        full twiddle tables.
+//   logN == 11         : one 2048-element tile per prime (R = 1).
 //   logN >= 12         : four-step, N = R x S with S = 2^min(11, logN - 6):
 //                        column pass (stages of distance >= S, along the R
 //                        rows of each column) and row pass (distance < S).
@@ -29,6 +30,8 @@ namespace fpm {
 //                        (N = 2^16, 2048-bit q: 180 us against 190 for 256 x 256,
 //                        N = 2^18: 758 against 960 for 512 x 512).
 constexpr uint32_t kSmallLogN = 10;
+// From here up they run as register-blocked rounds with tables of their own.
+constexpr uint32_t kWholeMinLogN = 8;
 constexpr uint32_t kTileLog = 11;            // 2048-element tiles
 constexpr uint32_t kTile = 1u << kTileLog;
 
