@@ -327,19 +327,19 @@ __global__ void __launch_bounds__(kThreads, 1)
         tc::mbar_init(sm.b_full, 1);
         for (int i = 0; i < 2; ++i) {
             tc::mbar_init(&sm.d_full[i], 1);
-            tc::mbar_init(&sm.d_empty[i], kCrtTile);
-            tc::mbar_init(&sm.m_full[i], kCrtTile);
-            tc::mbar_init(&sm.m_empty[i], kCrtTile);
+            tc::mbar_init(&sm.d_empty[i], kCrtTile / 32);
+            tc::mbar_init(&sm.m_full[i], kCrtTile / 32);
+            tc::mbar_init(&sm.m_empty[i], kCrtTile / 32);
         }
         for (uint32_t i = 0; i < ny; ++i) {
             tc::mbar_init(&sm.y_full[i], 1);
-            tc::mbar_init(&sm.y_empty[i], kStagers);
+            tc::mbar_init(&sm.y_empty[i], kStagers / 32);
         }
         for (uint32_t i = 0; i < na; ++i) {
-            tc::mbar_init(&sm.a_full[i], kStagers);
+            tc::mbar_init(&sm.a_full[i], kStagers / 32);
             tc::mbar_init(&sm.a_empty[i], 1);
         }
-        for (int i = 0; i < 8; ++i) tc::mbar_init(&sm.x_full[i], 32);
+        for (int i = 0; i < 8; ++i) tc::mbar_init(&sm.x_full[i], 1);
         *sm.abort = 0;
         tc::fence_mbar_init();
         // The constant image is read-only plan data: it loads under the
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 // Every value has been used, so its load is done: the box goes
                 // back (the fence orders these reads before the TMA's writes).
                 tc::fence_proxy_async_smem();
-                tc::mbar_arrive(&sm.y_empty[ys]);
+                tc::mbar_arrive_warp(&sm.y_empty[ys]);
                 if (++ys == ny) ys = 0, yph ^= 1;
                 // The operand slot is free once the MMAs of chunk g - na are done.
                 if (g >= na) {
@@ -528,10 +528,10 @@ __global__ void __launch_bounds__(kThreads, 1)
                     const float vh = (vf[0] + vf[1]) + (vf[2] + vf[3]);
                     sm.xch[xb * kCrtTile + m] = make_uint4(__float_as_uint(vh), static_cast<uint32_t>(t01),
                                                            static_cast<uint32_t>(t01 >> 32), t2);
-                    tc::mbar_arrive(&sm.x_full[2 * rw + xb]);
+                    tc::mbar_arrive_warp(&sm.x_full[2 * rw + xb]);
                 }
                 tc::fence_proxy_async_smem();
-                tc::mbar_arrive(&sm.a_full[as_]);
+                tc::mbar_arrive_warp(&sm.a_full[as_]);
                 if (++as_ == na) as_ = 0, aph ^= 1;
                 ++g;
             }
@@ -546,7 +546,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 // Top-limb sum as three words.
                 sm.meta[p * kCrtTile + m] =
                     make_uint4(static_cast<uint32_t>(t01), static_cast<uint32_t>(t01 >> 32), t2, 0u);
-                tc::mbar_arrive(&sm.m_full[p]);
+                tc::mbar_arrive_warp(&sm.m_full[p]);
             }
         }
     } else {
@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             const uint4 meta = sm.meta[grp * kCrtTile + row];
-            tc::mbar_arrive(&sm.m_empty[grp]);
+            tc::mbar_arrive_warp(&sm.m_empty[grp]);
             ok = tc::wait_or_abort(&sm.d_full[grp], k & 1, sm.abort, lim);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int64_t cy = ch.cy;
             // TMEM is read: the MMAs of this buffer's next tile may start.
             tc::tc_fence_before();
-            tc::mbar_arrive(&sm.d_empty[grp]);
+            tc::mbar_arrive_warp(&sm.d_empty[grp]);
             // r = X - e q in [-q, 2q): negative (cy < 0) adds q; a row near an
             // integer quotient subtracts q when r >= q (r past limb L - 1, or
             // its low L limbs at least q).  Rare: a second pass over the row.

@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         for (int i = 0; i < 2; ++i) {
             tc::mbar_init(&sm.d_full[i], 1);
-            tc::mbar_init(&sm.d_empty[i], kEpi);
+            tc::mbar_init(&sm.d_empty[i], kEpi / 32);
         }
         *sm.abort = 0;
         tc::fence_mbar_init();
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     hs[k][1] = rr[2] + (rr[3] << 8);
                 }
                 tc::tc_fence_before();
-                tc::mbar_arrive(&sm.d_empty[buf]);
+                tc::mbar_arrive_warp(&sm.d_empty[buf]);
                 // Byte offsets into the residues fit 32 bits (K N words below
                 // 2^30), one add a prime.
                 uint32_t at = (static_cast<uint32_t>(j0) * d.N + n0 + m) * 4u;

@@ -45,7 +45,9 @@ namespace {
 // S = 2^LOGS is a template parameter too, so a thread's strided global
 // accesses are one base address plus immediates.
 
-template <int LOGR, int LOGS, bool LAZY>
+// PDL: a kernel of the product's chain, which waits for the kernel before it
+// (pdl_wait) once its twiddles are on their way; the residues come after.
+template <int LOGR, int LOGS, bool LAZY, bool PDL = false>
 __device__ __forceinline__ void col_fwd_body(const DevPoint& d, uint32_t* A, uint32_t* B, int j, uint32_t bx) {
     extern __shared__ __align__(1024) uint32_t smem[];
     constexpr int RB = col_pass_rb(LOGR), E = 1 << RB, T = ntt_threads<RB>();
@@ -62,6 +64,7 @@ __device__ __forceinline__ void col_fwd_body(const DevPoint& d, uint32_t* A, uin
     const uint32_t p = d.pc[j].p;
     uint32_t* const X[2] = {A + j * N, B + j * N};
     for (uint32_t y = threadIdx.x; y < R; y += T) tw[y] = d.col_f[static_cast<size_t>(j) * R + y];
+    if constexpr (PDL) pdl_wait();
     const SharedTable table{tw};
     uint32_t* const tiles[2] = {ta, tb};
     {
@@ -86,7 +89,7 @@ __device__ __forceinline__ void col_fwd_body(const DevPoint& d, uint32_t* A, uin
     }
 }
 
-template <int LOGR, int LOGS, bool LAZY>
+template <int LOGR, int LOGS, bool LAZY, bool PDL = false>
 __device__ __forceinline__ void col_inv_body(const DevPoint& d, uint32_t* A, int j, uint32_t bx) {
     extern __shared__ __align__(1024) uint32_t smem[];
     constexpr int RB = col_pass_rb(LOGR), E = 1 << RB, T = ntt_threads<RB>();
@@ -102,6 +105,7 @@ __device__ __forceinline__ void col_inv_body(const DevPoint& d, uint32_t* A, int
     const uint32_t p = d.pc[j].p;
     uint32_t* const X[1] = {A + j * N};
     for (uint32_t y = threadIdx.x; y < R; y += T) tw[y] = d.col_i[static_cast<size_t>(j) * R + y];
+    if constexpr (PDL) pdl_wait();
     const SharedTable table{tw};
     {
         const uint32_t base = round_base<LOGR, XS, SWZ, RB, last>(threadIdx.x);
@@ -369,7 +373,7 @@ constexpr size_t row_bar_offset() {
 // count so far, mod 2); the barrier is initialised by the kernel.
 // smem: this team's region (row_smem_t<LOGS>() bytes, 1024-byte aligned);
 // tbar: its tables barrier (initialised, count 1).
-template <int LOGS, bool LAZY, class TEAM = BlockTeam>
+template <int LOGS, bool LAZY, class TEAM = BlockTeam, bool PDL = false>
 __device__ __forceinline__ void row_body(const DevPoint& d, uint32_t* A, uint32_t* B, int mode, int j, uint32_t bx,
                                          uint32_t phase, uint32_t* smem, uint64_t* tbar) {
     using RG = RowGeom<LOGS>;
@@ -392,6 +396,7 @@ __device__ __forceinline__ void row_body(const DevPoint& d, uint32_t* A, uint32_
 
     // The tables stream into shared memory while round 0 loads its elements.
     if (TEAM::tid() < 32) row_tables_bulk<LOGS>(tf, d, j, u0, tbar);
+    if constexpr (PDL) pdl_wait();
     // Round 0 straight from global memory (the thread's E elements lie in one
     // row).
     {
@@ -506,16 +511,14 @@ template <int LOGR, int LOGS, bool LAZY>
 __global__ void __launch_bounds__(col_threads<LOGR>(), (col_min_blocks<LOGR, 6>()))
     k_ntt_col_fwd(DevPoint d, uint32_t* A, uint32_t* B) {
     pdl_launch_dependents();
-    pdl_wait();
-    col_fwd_body<LOGR, LOGS, LAZY>(d, A, B, blockIdx.y, blockIdx.x);
+    col_fwd_body<LOGR, LOGS, LAZY, true>(d, A, B, blockIdx.y, blockIdx.x);
 }
 
 template <int LOGR, int LOGS, bool LAZY>
 __global__ void __launch_bounds__(col_threads<LOGR>(), (col_min_blocks<LOGR, 6>()))
     k_ntt_col_inv(DevPoint d, uint32_t* A) {
     pdl_launch_dependents();
-    pdl_wait();
-    col_inv_body<LOGR, LOGS, LAZY>(d, A, blockIdx.y, blockIdx.x);
+    col_inv_body<LOGR, LOGS, LAZY, true>(d, A, blockIdx.y, blockIdx.x);
 }
 
 template <int LOGS, bool LAZY>
@@ -528,8 +531,7 @@ __global__ void __launch_bounds__(row_threads<LOGS>(), (row_min_blocks<LOGS>()))
     }
     __syncthreads();
     pdl_launch_dependents();
-    pdl_wait();
-    row_body<LOGS, LAZY, BlockTeam>(d, A, B, mode, blockIdx.y, blockIdx.x, 0, smem, tbar);
+    row_body<LOGS, LAZY, BlockTeam, true>(d, A, B, mode, blockIdx.y, blockIdx.x, 0, smem, tbar);
 }
 
 // Grouped launches over products of one geometry class: a (possibly

@@ -40,6 +40,14 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(smem_addr(bar)) : "memory");
 }
 
+// One arrival for the whole (converged) warp, after what every lane did before.
+// Thirty-two lanes arriving one by one queue up on the barrier's word: the
+// barriers of a pipeline step count warps.
+__device__ __forceinline__ void mbar_arrive_warp(uint64_t* bar) {
+    __syncwarp();
+    if ((threadIdx.x & 31u) == 0) mbar_arrive(bar);
+}
+
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(smem_addr(bar)),
                  "r"(bytes)
