@@ -176,15 +176,6 @@ __device__ inline Smem carve(uint8_t* base, const Layout& lay) {
 
 static_assert(1 + 2 * kMaxSlots + 2 * kMaxASlots + 8 + 8 <= kBars, "barriers fit before tmem_base");
 
-// A shared load that the compiler may neither repeat nor move past the
-// barrier arrival that hands the slot back (a plain load may be done again
-// later instead of keeping its register, when TMA has refilled the slot).
-__device__ __forceinline__ uint32_t ld_shared_once(uint32_t addr) {
-    uint32_t x;
-    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(x) : "r"(addr) : "memory");
-    return x;
-}
-
 // Waits for this thread's TMEM loads; naming the registers keeps every read of
 // them below the wait.
 __device__ __forceinline__ void tmem_wait(uint32_t (&r)[16]) {
@@ -462,7 +453,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (!ok) break;
                 const uint32_t yrow = tc::smem_addr(sm.slot + ys * kSlot) + 4 * (h * kHalf * kCrtTile + m);
 #pragma unroll
-                for (int jj = 0; jj < kHalf; ++jj) yv[jj] = ld_shared_once(yrow + 4 * jj * kCrtTile);
+                for (int jj = 0; jj < kHalf; ++jj) yv[jj] = tc::ld_shared_once(yrow + 4 * jj * kCrtTile);
                 // Rows j >= K of the box read as zero and cf_j = 0 there, so
                 // every row of the chunk takes part without a test.
                 const uint4* kc = sm.kc + c * static_cast<int>(kChunk) + h * kHalf;

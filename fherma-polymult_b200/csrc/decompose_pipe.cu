@@ -11,20 +11,23 @@
 //     most 64 primes x 4 bytes x 4L bytes: at most 160 KB, resident in shared
 //     memory) and then, one thread, issues the MMAs, one chunk at a time: D
 //     goes to one of two 256-column TMEM buffers;
-//   * warps 1-4 copy each tile's limbs into a ring of two slots in the MMA's
-//     128-byte-swizzled K-major layout (the layout the tensor cores read at
-//     full rate) with asynchronous copies (cp.async) whose completion the
-//     slot's mbarrier tracks (cp.async.mbarrier.arrive), so a slot is handed
-//     to the MMAs the moment its copies land: a warp moves 8 rows x 4
-//     sixteen-byte groups at a time, so the global loads are 64-byte runs and
-//     the eight lanes of each shared-store phase hit eight different bank
-//     groups;
+//   * warps 1-4 bring each tile's limbs into a ring of operand slots in the
+//     MMA's 128-byte-swizzled K-major layout (the layout the tensor cores read at
+//     full rate).  Rows of whole 16-byte groups are copied there asynchronously
+//     (cp.async), the slot's mbarrier tracking the copies
+//     (cp.async.mbarrier.arrive), so a slot is handed to the MMAs the moment its
+//     copies land: a warp moves 8 rows x 4 groups at a time, so the global loads
+//     are 64-byte runs and the eight lanes of each shared-store phase hit eight
+//     different bank groups.  Other rows (RAW) arrive as whole tiles by bulk
+//     copies in a ring of their own and are moved to operand slots from there:
+//     copied word by word, by cp.async through L1, a pair took 20.1 us at L = 43,
+//     N = 65536 (17.6 now), 24.7 at L = 55 (23.4), 27.9 at L = 10, N = 2^18 (24.9);
 //   * warps 5-20, four per TMEM lane quadrant, one coefficient per thread,
 //     each take a quarter of a chunk's primes: read D, fold the 49-bit sums mod
 //     p_j and store the residues (a warp writes 32 consecutive words per
 //     prime).
-// The fold warps' instructions bound it (issue 54% active, tensor pipe 39%,
-// 106 MB in 25.3 us at K = 139, L = 64).  So every fold warp gets the same
+// What bounds it at L = 64 is the fold warps' way through a chunk: TMEM reads,
+// folds, stores (106 MB in 23.8 us at K = 139; 16 us without them).  So every fold warp gets the same
 // share of every chunk (K = 139 is 3 chunks of 48 with 12 primes a warp; as 64 +
 // 64 + 11, 16 a warp, the last chunk took as long as a full one), warps whose
 // rows and primes all exist store without a test per prime, and a store's
@@ -32,7 +35,8 @@
 // N = 65536 33.4 -> 25.3 us, K = 71 at N = 2^18 68.0 -> 47.6, K = 36 at
 // N = 2^17 21.7 -> 17.3, K = 60 at N = 32768 9.0 -> 8.2.  The fold constants
 // stay in the parameter bank: from shared memory, which the MMAs load heavily,
-// they took K = 60 from 8.2 to 9.1 us (and K = 139 from 25.3 to 24.4).
+// they took K = 60 from 8.2 to 9.1 us (and K = 139 from 25.3 to 24.4).  (Figures
+// of that step; the ring's and the fold's are beside them below.)
 // The fold constants come from kernel parameters.  Every wait is bounded
 // (DevPoint::wait_ns); a timeout raises an abort flag that every role checks,
 // and the error word gets bit 0.
@@ -40,6 +44,8 @@
 #include "kernels.h"
 #include "pdl.cuh"
 #include "tc.cuh"
+
+#include <algorithm>
 
 namespace fpm {
 
@@ -51,6 +57,9 @@ constexpr int kLoaders = 128;
 constexpr int kEpiWarp0 = 5;                       // warps 5-20
 constexpr int kEpi = 512;
 constexpr uint32_t kRows = 128;
+constexpr uint32_t kMaxSlots = 8;                  // operand tiles in their ring
+constexpr uint32_t kMaxRaw = 8;                    // raw tiles in theirs
+constexpr uint32_t kBars = 1 + 2 * kMaxSlots + 2 * kMaxRaw + 4;
 constexpr uint32_t kBufCols = 256;                 // TMEM columns of one of the two buffers
 
 // Operand tiles and the constant image in the 128-byte-swizzle layout
@@ -60,33 +69,67 @@ __host__ __device__ inline uint32_t a_bytes(uint32_t kb) { return static_cast<ui
 __host__ __device__ inline size_t b_bytes(uint32_t kb, int nch, uint32_t cols) {
     return static_cast<size_t>(nch) * sw128_bytes(cols, kb);
 }
-__host__ inline size_t smem_bytes(uint32_t kb, int nch, uint32_t cols) {
-    return b_bytes(kb, nch, cols) + 2 * a_bytes(kb) + 128;
+constexpr size_t kSmemLimit = 227 * 1024;
+
+// The rings: `slots` operand tiles, and for rows that are not whole 16-byte
+// groups (L not a multiple of 4) `raw` tiles as they lie in memory (128 L words).
+struct Rings {
+    uint32_t slots, raw;
+};
+__host__ __device__ inline uint32_t raw_bytes(int L) { return kRows * 4 * static_cast<uint32_t>(L); }
+__host__ inline size_t smem_bytes(uint32_t kb, int nch, uint32_t cols, int L, Rings r) {
+    return b_bytes(kb, nch, cols) + r.slots * size_t(a_bytes(kb)) + r.raw * size_t(raw_bytes(L)) + kBars * 8 + 16;
+}
+// Whole 16-byte groups are copied straight into operand slots, so every slot is
+// a tile in flight: as many as shared memory holds beside the constants, 2 to
+// kMaxSlots.  A tile's limbs are about 2 us away once the pipelines run, and two
+// 16 KB tiles held a CTA to one a microsecond: a pair with more slots than two
+// takes 44.1 us for 47.4 (L = 32, K = 71, N = 2^18), 15.0 for 17.3 (L = 16,
+// K = 36, N = 2^17); L = 64 has room for two.  Other rows wait in the raw ring, four
+// tiles or more of it before a third operand slot.  Without room for a raw tile
+// they are copied word by word.
+__host__ inline Rings ring_sizes(uint32_t kb, int nch, uint32_t cols, int L) {
+    Rings r{2, 0};
+    if (L & 3) {
+        r = Rings{4, kMaxRaw};
+        while (r.raw > 4 && smem_bytes(kb, nch, cols, L, r) > kSmemLimit) --r.raw;
+        while (r.slots > 2 && smem_bytes(kb, nch, cols, L, r) > kSmemLimit) --r.slots;
+        while (r.raw > 0 && smem_bytes(kb, nch, cols, L, r) > kSmemLimit) --r.raw;
+    } else {
+        r.slots = kMaxSlots;
+        while (r.slots > 2 && smem_bytes(kb, nch, cols, L, r) > kSmemLimit) --r.slots;
+    }
+    return r;
 }
 
 struct Smem {
     uint8_t* b;            // resident constant image
-    uint8_t* a;            // [2] operand tiles
+    uint8_t* a;            // [slots] operand tiles
+    uint8_t* raw;          // [raw] tiles as they lie in memory
     uint64_t* b_full;      // [1]
-    uint64_t* a_full;      // [2]
-    uint64_t* a_empty;     // [2]
+    uint64_t* a_full;      // [kMaxSlots]
+    uint64_t* a_empty;     // [kMaxSlots]
+    uint64_t* r_full;      // [kMaxRaw] a raw tile landed
+    uint64_t* r_empty;     // [kMaxRaw] and the loaders have read it
     uint64_t* d_full;      // [2]
     uint64_t* d_empty;     // [2]
     uint32_t* tmem_base;
     volatile uint32_t* abort;
 };
 
-__device__ inline Smem carve(uint8_t* base, uint32_t kb, int nch, uint32_t cols) {
+__device__ inline Smem carve(uint8_t* base, uint32_t kb, int nch, uint32_t cols, int L, Rings rings) {
     Smem s;
     s.b = base;
     s.a = base + b_bytes(kb, nch, cols);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(s.a + 2 * a_bytes(kb));
-    s.b_full = bars;
-    s.a_full = bars + 1;
-    s.a_empty = bars + 3;
-    s.d_full = bars + 5;
-    s.d_empty = bars + 7;
-    s.tmem_base = reinterpret_cast<uint32_t*>(bars + 9);
+    s.raw = s.a + rings.slots * a_bytes(kb);
+    s.b_full = reinterpret_cast<uint64_t*>(s.raw + rings.raw * raw_bytes(L));
+    s.a_full = s.b_full + 1;
+    s.a_empty = s.a_full + kMaxSlots;
+    s.r_full = s.a_empty + kMaxSlots;
+    s.r_empty = s.r_full + kMaxRaw;
+    s.d_full = s.r_empty + kMaxRaw;
+    s.d_empty = s.d_full + 2;
+    s.tmem_base = reinterpret_cast<uint32_t*>(s.b_full + kBars);
     s.abort = s.tmem_base + 1;
     return s;
 }
@@ -136,30 +179,41 @@ __device__ __forceinline__ void tmem_read(uint32_t taddr, uint32_t (&r)[NC]) {
 
 // A GEMM sum D is below 4L 255^2 <= 256 * 65025 (L <= 64), so both halves of
 // sum_s D_s 2^(8s), A = D_0 + 2^8 D_1 and B = D_2 + 2^8 D_3, are below
-// 257 * 256 * 65025 < 2^32, and the residue is (A + B 2^16) mod p:
-// f = {p, 2^16 mod p, its Shoup companion, floor(2^32 / p)}.  LAZY leaves a
-// value below 4p, congruent to the same residue, for a transform whose first
-// butterflies take lazy input.
+// 257 * 256 * 65025 < 2^32, and the residue is X = A + 2^16 B mod p, X < 2^48.1.
 static_assert(kMaxL <= 64, "D_0 + 2^8 D_1 must fit 32 bits");
-template <bool LAZY>
+// Canonical: f = {p, 2^16 mod p, its Shoup companion, floor(2^32 / p)}.
 __device__ __forceinline__ uint32_t fold_halves(uint32_t A, uint32_t B, uint4 f) {
+    return add_mod(shoup(A, 1u, f.w, f.x), shoup(B, f.y, f.z, f.x), f.x);
+}
+// A value below 2p, congruent to the residue, for a transform whose first
+// butterflies take lazy input: f = {p, mu = floor(2^49 / p)}.  With
+// t = floor(B / 2) + floor(A / 2^17) > X / 2^17 - 1.5 the quotient estimate
+// floor(t mu / 2^32) is at most X / p and above X / p - X / 2^49 - 1.5 2^17 / p
+// - 1, so more than X / p - 1.6 (p > 2^24).  One high product and one low one,
+// where a Shoup quotient for each half took two of each on the pipe that
+// multiplies: 44.1 -> 40.7 us for a pair at N = 2^18, K = 71, L = 32, 15.0 ->
+// 14.6 at N = 2^17, K = 36, L = 16.
+__device__ __forceinline__ uint32_t fold_halves(uint32_t A, uint32_t B, uint2 f) {
+    const uint32_t q = mulhi32((B >> 1) + (A >> 17), f.y);
+    return A + (B << 16) - q * f.x;
+}
+template <bool LAZY>
+__device__ __forceinline__ auto fold_consts(const DecConsts& fc, int j) {
     if constexpr (LAZY) {
-        // (A - q1 p) + (B f.y - q2 p), each term in [0, 2p) (Shoup): one
-        // product by p for both quotients, the same value below 4p.
-        const uint32_t q = mulhi32(A, f.w) + mulhi32(B, f.z);
-        return B * f.y + A - q * f.x;
+        return fc.lazy[j];
     } else {
-        return add_mod(shoup(A, 1u, f.w, f.x), shoup(B, f.y, f.z, f.x), f.x);
+        return fc.fold[j];
     }
 }
 
 // CTAs [0, split) take operand 0 (la -> ra), [split, gridDim.x) operand 1.
 // P: primes per fold warp and chunk.
-template <int P, bool LAZY>
+// RAW: rows that are not whole 16-byte groups, in a raw ring.
+template <int P, bool LAZY, bool RAW>
 __global__ void __launch_bounds__(kThreads, 1)
     k_decompose_pipe(DevPoint d, const __grid_constant__ DecConsts fc, const uint32_t* __restrict__ la,
                      const uint32_t* __restrict__ lb, uint32_t* __restrict__ ra, uint32_t* __restrict__ rb,
-                     int operand0, uint32_t n_begin, uint32_t n_end, uint32_t split) {
+                     int operand0, uint32_t n_begin, uint32_t n_end, uint32_t split, Rings rings) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     pdl_launch_dependents();
     // The 128-byte swizzle is a function of the shared address: the
@@ -171,10 +225,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t kb = d.dec_kb;
     const int nch = static_cast<int>(fc.chunks);
     constexpr uint32_t cols = 16 * P;
-    const Smem sm = carve(smem_raw, kb, nch, cols);
-    // (The shuffle tells the compiler that the warp index is uniform.)
+        // (The shuffle tells the compiler that the warp index is uniform.)
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int L = d.L, K = d.K;
+    const Smem sm = carve(smem_raw, kb, nch, cols, L, rings);
+    const uint32_t slots = rings.slots;
     const bool second = blockIdx.x >= split;
     const int operand = operand0 + (second ? 1 : 0);
     const uint32_t* limbs = second ? lb : la;
@@ -187,13 +242,17 @@ __global__ void __launch_bounds__(kThreads, 1)
 
     if (threadIdx.x == 0) {
         tc::mbar_init(sm.b_full, 1);
-        for (int i = 0; i < 2; ++i) {
+        for (uint32_t i = 0; i < slots; ++i) {
             tc::mbar_init(&sm.a_full[i], kLoaders);
             tc::mbar_init(&sm.a_empty[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
             tc::mbar_init(&sm.d_full[i], 1);
             tc::mbar_init(&sm.d_empty[i], kEpi / 32);
+        }
+        for (uint32_t i = 0; RAW && i < rings.raw; ++i) {
+            tc::mbar_init(&sm.r_full[i], 1);
+            tc::mbar_init(&sm.r_empty[i], kLoaders / 32);
         }
         *sm.abort = 0;
         tc::fence_mbar_init();
@@ -222,10 +281,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             bool ok = tc::wait_or_abort(sm.b_full, 0, sm.abort, lim);
             uint64_t* last_bar = nullptr;   // the barrier of the latest commit
             uint32_t last_par = 0;
-            uint32_t g = 0, i = 0;
-            for (uint32_t t = blockIdx.x - g0; ok && t < tiles; t += gs, ++i) {
-                const int s = i & 1;
-                ok = tc::wait_or_abort(&sm.a_full[s], (i >> 1) & 1, sm.abort, lim);
+            uint32_t g = 0, s = 0, ph = 0;   // chunk count; operand slot and its phase
+            for (uint32_t t = blockIdx.x - g0; ok && t < tiles; t += gs) {
+                ok = tc::wait_or_abort(&sm.a_full[s], ph, sm.abort, lim);
                 if (!ok) break;
                 // The limbs came through the generic proxy (cp.async).
                 tc::fence_proxy_async_smem();
@@ -251,12 +309,74 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (!ok) break;
                 tc::mma_commit(&sm.a_empty[s]);
                 last_bar = &sm.a_empty[s];
-                last_par = (i >> 1) & 1;
+                last_par = ph;
+                if (++s == slots) s = 0, ph ^= 1;
             }
             // MMAs still running must finish before the CTA may exit.
             if (last_bar) tc::wait_parity(last_bar, last_par, lim);
             // So must the constant image, if an abort came before it landed.
             if (!(d.fault & kFaultDecompose)) tc::wait_parity(sm.b_full, 0, lim);
+        }
+        __syncwarp();
+    } else if (RAW && warp < kEpiWarp0 && (reinterpret_cast<uintptr_t>(limbs) & 15u) == 0 &&
+               (((n_end - n_begin) * static_cast<uint32_t>(L)) & 3u) == 0) {
+        // ---- loaders, rows that are not whole 16-byte groups: a tile arrives
+        // as it lies in memory, one bulk copy (its rows are contiguous and, 128
+        // rows a tile, start and end on 16 bytes); a thread then moves one row
+        // to the operand slot, word by word out (lanes L words apart), 16
+        // bytes at a time in.
+        const uint32_t m = threadIdx.x - kLoadWarp0 * 32;
+        const uint32_t G = kb / 16;
+        uint32_t s = 0, ph = 0, rs = 0, rph = 0, i = 0;
+        // Lane 0 of the first loader warp requests the tiles, rings.raw ahead.
+        const bool asks = m == 0;
+        uint32_t ask_t = blockIdx.x - g0, asked = 0;
+        auto ask = [&](uint32_t slot) {
+            const uint32_t r0 = n_begin + ask_t * kRows;
+            const uint32_t bytes = min(kRows, n_end - r0) * 4 * static_cast<uint32_t>(L);
+            tc::mbar_arrive_expect_tx(&sm.r_full[slot], bytes);
+            tc::bulk_g2s(sm.raw + slot * raw_bytes(L), limbs + static_cast<size_t>(r0) * L, bytes, &sm.r_full[slot]);
+            ask_t += gs;
+            ++asked;
+        };
+        if (asks)
+            for (uint32_t k = 0; k < rings.raw && ask_t < tiles; ++k) ask(k);
+        __syncwarp();
+        bool ok = true;
+        for (uint32_t t = blockIdx.x - g0; t < tiles; t += gs, ++i) {
+            const uint32_t nk = min(kRows, n_end - (n_begin + t * kRows));
+            ok = tc::wait_or_abort(&sm.r_full[rs], rph, sm.abort, lim);
+            if (ok && i >= slots) ok = tc::wait_or_abort(&sm.a_empty[s], ph ^ 1, sm.abort, lim);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            const uint32_t row = tc::smem_addr(sm.raw + rs * raw_bytes(L)) + m * 4 * static_cast<uint32_t>(L);
+            uint8_t* at = sm.a + s * a_bytes(kb);
+#pragma unroll 4
+            for (uint32_t gq = 0; gq < G; ++gq) {
+                uint32_t w[4];
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k)
+                    w[k] = m < nk && 4 * gq + k < static_cast<uint32_t>(L) ? tc::ld_shared_once(row + 16 * gq + 4 * k) : 0u;
+                *reinterpret_cast<uint4*>(at + sw128_offset(m, 16 * gq, kRows)) = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+            // The row is written (to the MMAs) and read (back to the copies).
+            tc::fence_proxy_async_smem();
+            tc::mbar_arrive(&sm.a_full[s]);
+            tc::mbar_arrive_warp(&sm.r_empty[rs]);
+            if (asks && ask_t < tiles) {
+                ok = tc::wait_or_abort(&sm.r_empty[rs], rph, sm.abort, lim);
+                if (ok) ask(rs);
+            }
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            if (++s == slots) s = 0, ph ^= 1;
+            if (++rs == rings.raw) rs = 0, rph ^= 1;
+        }
+        // Every copy asked for lands before the CTA may exit.
+        if (asks) {
+            const uint32_t from = asked > rings.raw ? asked - rings.raw : 0;
+            for (uint32_t k = from; k < asked; ++k)
+                tc::wait_parity(&sm.r_full[k % rings.raw], (k / rings.raw) & 1, lim);
         }
         __syncwarp();
     } else if (warp < kEpiWarp0) {
@@ -271,12 +391,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t G = kb / 16;                    // 16-byte K groups per row
         const uint32_t r = lane & 7, gi = lane >> 3;   // row in block, group (or limb) in block
         const uint32_t gbs = (G + 3) / 4;
-        uint32_t i = 0;
+        uint32_t i = 0, s = 0, ph = 0;
         bool ok = true;
         for (uint32_t t = blockIdx.x - g0; t < tiles; t += gs, ++i) {
-            const int s = i & 1;
-            if (i >= 2) {
-                ok = tc::wait_or_abort(&sm.a_empty[s], ((i - 2) >> 1) & 1, sm.abort, lim);
+            if (i >= slots) {
+                ok = tc::wait_or_abort(&sm.a_empty[s], ph ^ 1, sm.abort, lim);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
             }
@@ -310,6 +429,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             // the next slot at once; the MMA issuer fences the async proxy.
             cp_async_commit();
             cp_async_arrive_noinc(&sm.a_full[s]);
+            if (++s == slots) s = 0, ph ^= 1;
         }
         // Whatever is still in flight lands before the CTA may exit.
         cp_async_wait<0>();
@@ -353,7 +473,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (whole && j0 + P <= K) {
 #pragma unroll
                     for (int k = 0; k < P; ++k) {
-                        *reinterpret_cast<uint32_t*>(out + at) = fold_halves<LAZY>(hs[k][0], hs[k][1], fc.fold[j0 + k]);
+                        *reinterpret_cast<uint32_t*>(out + at) = fold_halves(hs[k][0], hs[k][1], fold_consts<LAZY>(fc, j0 + k));
                         at += stride;
                     }
                 } else {
@@ -361,7 +481,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     for (int k = 0; k < P; ++k) {
                         if (live && j0 + k < K)
                             *reinterpret_cast<uint32_t*>(out + at) =
-                                fold_halves<LAZY>(hs[k][0], hs[k][1], fc.fold[j0 + k]);
+                                fold_halves(hs[k][0], hs[k][1], fold_consts<LAZY>(fc, j0 + k));
                         at += stride;
                     }
                 }
@@ -383,33 +503,40 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 DecConsts make_dec_consts(const HostPlan& pl, const uint8_t* img_a, const uint8_t* img_b) {
     DecConsts dc{};
-    for (int j = 0; j < pl.K; ++j) dc.fold[j] = pl.dec_fold[j];
     dc.img[0] = img_a;
     dc.img[1] = img_b;
     dc.chunks = pl.dec_wchunks;
     dc.piece = pl.dec_wpiece;
     // The four-step transforms start with lazy butterflies; the one-block
     // transform (N <= 1024) and the full-reduction window want canonical input.
-    dc.lazy_out = pl.lazy && pl.g.logN > kSmallLogN ? 1u : 0u;
+    dc.lazy_out = pl.lazy && pl.g.logN > kSmallLogN && *std::min_element(pl.primes.begin(), pl.primes.end()) > (1u << 24);
+    for (int j = 0; j < pl.K; ++j) {
+        if (dc.lazy_out) {
+            const uint32_t p = pl.primes[j];
+            dc.lazy[j] = make_uint2(p, static_cast<uint32_t>((1ull << 49) / p));
+        } else {
+            dc.fold[j] = pl.dec_fold[j];
+        }
+    }
     return dc;
 }
 
 namespace {
 
 using DecKernel = void (*)(DevPoint, const DecConsts, const uint32_t*, const uint32_t*, uint32_t*, uint32_t*, int,
-                           uint32_t, uint32_t, uint32_t);
+                           uint32_t, uint32_t, uint32_t, Rings);
 
-template <bool LAZY>
+template <bool LAZY, bool RAW>
 DecKernel dec_kernel(uint32_t piece) {
     switch (piece) {
-        case 2: return k_decompose_pipe<2, LAZY>;
-        case 4: return k_decompose_pipe<4, LAZY>;
-        case 6: return k_decompose_pipe<6, LAZY>;
-        case 8: return k_decompose_pipe<8, LAZY>;
-        case 10: return k_decompose_pipe<10, LAZY>;
-        case 12: return k_decompose_pipe<12, LAZY>;
-        case 14: return k_decompose_pipe<14, LAZY>;
-        case 16: return k_decompose_pipe<16, LAZY>;
+        case 2: return k_decompose_pipe<2, LAZY, RAW>;
+        case 4: return k_decompose_pipe<4, LAZY, RAW>;
+        case 6: return k_decompose_pipe<6, LAZY, RAW>;
+        case 8: return k_decompose_pipe<8, LAZY, RAW>;
+        case 10: return k_decompose_pipe<10, LAZY, RAW>;
+        case 12: return k_decompose_pipe<12, LAZY, RAW>;
+        case 14: return k_decompose_pipe<14, LAZY, RAW>;
+        case 16: return k_decompose_pipe<16, LAZY, RAW>;
         default: throw std::runtime_error("decompose: unsupported chunk size");
     }
 }
@@ -418,13 +545,14 @@ DecKernel dec_kernel(uint32_t piece) {
 
 bool decompose_pipe_supported(const HostPlan& pl) {
     return pl.K <= kMaxK && pl.dec_wchunks >= 1 && pl.dec_wpiece >= 2 && pl.dec_wpiece <= 16 &&
-           smem_bytes(pl.dec_kb, static_cast<int>(pl.dec_wchunks), 16 * pl.dec_wpiece) <= 227 * 1024;
+           smem_bytes(pl.dec_kb, static_cast<int>(pl.dec_wchunks), 16 * pl.dec_wpiece, pl.L, Rings{2, 0}) <= kSmemLimit;
 }
 
 void decompose_pipe_init_attributes() {
     for (uint32_t piece = 2; piece <= 16; piece += 2)
-        for (DecKernel k : {dec_kernel<false>(piece), dec_kernel<true>(piece)})
-            check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024),
+        for (DecKernel k : {dec_kernel<false, false>(piece), dec_kernel<false, true>(piece),
+                            dec_kernel<true, false>(piece), dec_kernel<true, true>(piece)})
+            check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemLimit)),
                   "decompose_pipe smem");
 }
 
@@ -440,9 +568,14 @@ void launch_decompose_pipe(const DevPoint& d, const DecConsts& dc, const uint32_
     if (per > tiles) per = tiles;
     const uint32_t grid = per * operands;
     const uint32_t split = operands == 2 ? per : grid;
-    check(launch_pdl(dc.lazy_out ? dec_kernel<true>(dc.piece) : dec_kernel<false>(dc.piece), dim3(grid),
-                     dim3(kThreads), smem_bytes(d.dec_kb, static_cast<int>(dc.chunks), 16 * dc.piece), st, d, dc, a,
-                     b ? b : a, A, B ? B : A, operand0, n_begin, n_end, split),
+    const int nch = static_cast<int>(dc.chunks);
+    const uint32_t cols = 16 * dc.piece;
+    const Rings rings = ring_sizes(d.dec_kb, nch, cols, d.L);
+    const DecKernel kernel =
+        rings.raw ? (dc.lazy_out ? dec_kernel<true, true>(dc.piece) : dec_kernel<false, true>(dc.piece))
+                  : (dc.lazy_out ? dec_kernel<true, false>(dc.piece) : dec_kernel<false, false>(dc.piece));
+    check(launch_pdl(kernel, dim3(grid), dim3(kThreads), smem_bytes(d.dec_kb, nch, cols, d.L, rings), st, d, dc, a, b ? b : a, A,
+                     B ? B : A, operand0, n_begin, n_end, split, rings),
           "decompose launch");
 }
 

@@ -112,7 +112,12 @@ void launch_crt_pipe(const DevPoint& d, const CrtConsts& cc, const uint32_t* Y, 
 // b != nullptr the CTAs split between a -> A (operand 0) and b -> B (1),
 // otherwise all take a -> A as operand `operand0`.
 struct DecConsts {
-    uint4 fold[kMaxK];          // {p, 2^16 mod p, its Shoup companion, floor(2^32 / p)}
+    // Fold constants: {p, 2^16 mod p, its Shoup companion, floor(2^32 / p)}, or
+    // with lazy_out {p, floor(2^49 / p)}.
+    union {
+        uint4 fold[kMaxK];
+        uint2 lazy[kMaxK];
+    };
     const uint8_t* img[2];      // device copies of the plan's wide images, operands a and b
     uint32_t chunks;            // chunks of 4 piece primes (16 piece GEMM columns)
     uint32_t piece;             // primes per fold warp and chunk: 2, 4 .. 16

@@ -118,6 +118,15 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
         : "memory");
 }
 
+// A shared load that the compiler may neither repeat nor move past the
+// barrier arrival that hands the slot back (a plain load may be done again
+// later instead of keeping its register, when the next copy has refilled the slot).
+__device__ __forceinline__ uint32_t ld_shared_once(uint32_t addr) {
+    uint32_t x;
+    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(x) : "r"(addr) : "memory");
+    return x;
+}
+
 // 2-D tensor copies through a tensor map (tmap.h) of this GPU's memory.  x is
 // the column (word) coordinate, y the row; x * 4 bytes must be a multiple of
 // 16.  The map lives in kernel-parameter space (__grid_constant__).
