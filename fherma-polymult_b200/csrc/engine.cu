@@ -1,10 +1,11 @@
 // Engine: plan upload, buffers, and the launch sequence of one product.
 //
 // Reference counterpart: fherma_init / fherma_run / fherma_free,
-// solve.cu:710-1083.  The product is four launches on one stream: decompose a,
-// decompose b (scaled), the transform chain (column pass, fused row pass,
-// inverse column pass), CRT.  The host path stages the caller's buffers
-// through pinned memory in chunks so the copies overlap the host-side memcpys.
+// solve.cu:710-1083.  The product is three to five launches on one stream:
+// decompose a and b (scaled), the transform chain (one launch where it fits the
+// GPU at once, else column pass, fused row pass, inverse column pass), CRT.  The
+// host path stages a caller's pageable buffers through pinned memory in chunks
+// so the copies overlap the host-side memcpys.
 #include "engine.h"
 #include "kernels.h"
 
@@ -257,7 +258,8 @@ void Engine::release() {
     for (uint32_t* h : {ha_, hb_, hc_}) {
         if (h) cudaFreeHost(h);
     }
-    ha_ = hb_ = hc_ = nullptr;
+    if (herr_) cudaFreeHost(herr_);
+    ha_ = hb_ = hc_ = herr_ = nullptr;
 }
 
 void Engine::launch_dec(const uint32_t* d_limbs, uint32_t* d_res, int operand, uint32_t n0, uint32_t n1,
@@ -358,12 +360,9 @@ bool is_pinned(const void* p) {
 void Engine::ensure_host_path() {
     if (la_) return;
     const size_t n = words(), bytes = n * sizeof(uint32_t);
-    la_ = dalloc<uint32_t>(n);
-    lb_ = dalloc<uint32_t>(n);
+    if (!herr_) check(cudaHostAlloc(reinterpret_cast<void**>(&herr_), sizeof(uint32_t), cudaHostAllocDefault), "pinned");
     lc_ = dalloc<uint32_t>(n);
-    check(cudaHostAlloc(reinterpret_cast<void**>(&ha_), bytes, cudaHostAllocDefault), "pinned");
-    check(cudaHostAlloc(reinterpret_cast<void**>(&hb_), bytes, cudaHostAllocDefault), "pinned");
-    check(cudaHostAlloc(reinterpret_cast<void**>(&hc_), bytes, cudaHostAllocDefault), "pinned");
+    lb_ = dalloc<uint32_t>(n);
     // I/O chunks: equal slices on 128-coefficient boundaries, so a chunk's
     // decompose and CRT blocks never straddle two.  Each chunk costs about
     // 13 us of launches and pipeline start-up, so the default aims at 16 MiB of
@@ -373,7 +372,16 @@ void Engine::ensure_host_path() {
     int want = static_cast<int>(std::min<size_t>(4, std::max<size_t>(1, (in_bytes + (size_t(8) << 20)) >> 24)));
     if (const char* v = std::getenv("FPM_IO_CHUNKS")) want = std::max(1, std::atoi(v));
     set_chunks(want);
-    pool_.reset(new CopyPool(default_copy_threads()));
+    la_ = dalloc<uint32_t>(n);   // last: what says that all of the above is there
+}
+
+// The pinned staging buffer `h` and the copy threads, for a caller's pageable
+// buffer (pinned ones are copied from and to directly: their first product used
+// to wait 36 ms at N = 65536, W = 2048 for staging it never touched).
+uint32_t* Engine::staging(uint32_t*& h) {
+    if (!h) check(cudaHostAlloc(reinterpret_cast<void**>(&h), words() * sizeof(uint32_t), cudaHostAllocDefault), "pinned");
+    if (!pool_) pool_.reset(new CopyPool(default_copy_threads()));
+    return h;
 }
 
 void Engine::set_chunks(int want) {
@@ -399,6 +407,7 @@ int Engine::tune_host_path() {
     if (std::getenv("FPM_IO_CHUNKS")) return static_cast<int>(chunk_at_.size() - 1);
     const int dflt = static_cast<int>(chunk_at_.size() - 1);
     const size_t bytes = words() * sizeof(uint32_t);
+    for (uint32_t** h : {&ha_, &hb_, &hc_}) staging(*h);
     std::memset(ha_, 0, bytes);
     std::memset(hb_, 0, bytes);
     auto time_it = [&](int n) {
@@ -436,6 +445,9 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c, uint32_
     cudaEvent_t* in_ev = events_.data();              // 2 nch
     cudaEvent_t* crt_ev = events_.data() + 2 * nch;   // nch
     cudaEvent_t* out_ev = events_.data() + 3 * nch;   // nch
+    if (!pin_a) staging(ha_);
+    if (!pin_b) staging(hb_);
+    if (!pin_c) staging(hc_);
 
     // In: per chunk, (stage,) DMA, then that chunk's decompose.
     const uint32_t* src[2] = {a, b};
@@ -443,32 +455,54 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c, uint32_
     uint32_t* stage[2] = {ha_, hb_};
     uint32_t* dlimbs[2] = {la_, lb_};
     uint32_t* res[2] = {A_, B_};
-    for (int op = 0; op < 2; ++op) {
+    auto bring_in = [&](int op, size_t off, size_t bytes, cudaStream_t st) {
+        const uint32_t* from = src[op] + off;
+        if (!pinned[op]) {
+            pool_->copy(stage[op] + off, from, bytes);
+            from = stage[op] + off;
+        }
+        check(cudaMemcpyAsync(dlimbs[op] + off, from, bytes, cudaMemcpyHostToDevice, st), "copy in");
+    };
+    uint32_t* dst = pin_c ? c : hc_;
+    // A small product is one stream's work: both copies in, the device
+    // product with its paired decompose, the copy out.  An operand of 256 KiB
+    // is 5 us of DMA, less than the second decompose launch and the events
+    // between streams take (N = 4096, W = 256 from pageable arrays: 88 us
+    // with them, 65 without, the error word's own synchronous copy
+    // included).
+    const size_t all = words() * sizeof(uint32_t);
+    const bool small = nch == 1 && all <= (size_t(256) << 10);
+    if (small) {
+        for (int op = 0; op < 2; ++op) bring_in(op, 0, all, stream_);
+        product(dp_, la_, lb_, A_, B_, lc_, stream_);
+        check(cudaMemcpyAsync(dst, lc_, all, cudaMemcpyDeviceToHost, stream_), "copy out");
+        check(cudaMemcpyAsync(herr_, dp_.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream_), "read error word");
+        check(cudaEventRecord(out_ev[0], stream_), "event");
+    } else {
+        for (int op = 0; op < 2; ++op) {
+            for (size_t k = 0; k < nch; ++k) {
+                const uint32_t n0 = chunk_at_[k], n1 = chunk_at_[k + 1];
+                const size_t off = static_cast<size_t>(n0) * L, bytes = static_cast<size_t>(n1 - n0) * L * 4;
+                bring_in(op, off, bytes, copy_);
+                check(cudaEventRecord(in_ev[op * nch + k], copy_), "event");
+                check(cudaStreamWaitEvent(stream_, in_ev[op * nch + k], 0), "wait");
+                launch_dec(dlimbs[op], res[op], op, n0, n1, stream_);
+            }
+        }
+        launch_ntt(dp_, A_, B_, kRowProduct, stream_);
+        // Out: per chunk, the CRT, then its DMA (to c itself when c is
+        // pinned); the error word goes out behind the last one.
         for (size_t k = 0; k < nch; ++k) {
             const uint32_t n0 = chunk_at_[k], n1 = chunk_at_[k + 1];
             const size_t off = static_cast<size_t>(n0) * L, bytes = static_cast<size_t>(n1 - n0) * L * 4;
-            const uint32_t* from = src[op] + off;
-            if (!pinned[op]) {
-                pool_->copy(stage[op] + off, from, bytes);
-                from = stage[op] + off;
-            }
-            check(cudaMemcpyAsync(dlimbs[op] + off, from, bytes, cudaMemcpyHostToDevice, copy_), "copy in");
-            check(cudaEventRecord(in_ev[op * nch + k], copy_), "event");
-            check(cudaStreamWaitEvent(stream_, in_ev[op * nch + k], 0), "wait");
-            launch_dec(dlimbs[op], res[op], op, n0, n1, stream_);
+            launch_crt_any(dp_, A_, lc_, n0, n1, stream_);
+            check(cudaEventRecord(crt_ev[k], stream_), "event");
+            check(cudaStreamWaitEvent(out_, crt_ev[k], 0), "wait");
+            check(cudaMemcpyAsync(dst + off, lc_ + off, bytes, cudaMemcpyDeviceToHost, out_), "copy out");
+            if (k + 1 == nch)
+                check(cudaMemcpyAsync(herr_, dp_.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, out_), "read error word");
+            check(cudaEventRecord(out_ev[k], out_), "event");
         }
-    }
-    launch_ntt(dp_, A_, B_, kRowProduct, stream_);
-    // Out: per chunk, the CRT, then its DMA (to c itself when c is pinned).
-    uint32_t* dst = pin_c ? c : hc_;
-    for (size_t k = 0; k < nch; ++k) {
-        const uint32_t n0 = chunk_at_[k], n1 = chunk_at_[k + 1];
-        const size_t off = static_cast<size_t>(n0) * L, bytes = static_cast<size_t>(n1 - n0) * L * 4;
-        launch_crt_any(dp_, A_, lc_, n0, n1, stream_);
-        check(cudaEventRecord(crt_ev[k], stream_), "event");
-        check(cudaStreamWaitEvent(out_, crt_ev[k], 0), "wait");
-        check(cudaMemcpyAsync(dst + off, lc_ + off, bytes, cudaMemcpyDeviceToHost, out_), "copy out");
-        check(cudaEventRecord(out_ev[k], out_), "event");
     }
     check(cudaGetLastError(), "product launch");
     if (!c) c = out_fn(out_arg);
@@ -482,7 +516,8 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c, uint32_
     } else {
         check(cudaEventSynchronize(out_ev[nch - 1]), "copy out");
     }
-    if (const uint32_t e = take_error()) {
+    if (const uint32_t e = *herr_) {
+        check(cudaMemset(dp_.err, 0, sizeof(uint32_t)), "clear error word");
         throw PipelineTimeout("a kernel pipeline wait ran out of time (error word " + std::to_string(e) +
                               "); this product's result is not valid");
     }

@@ -110,6 +110,7 @@ private:
     void launch_crt_any(const DevPoint& d, const uint32_t* d_y, uint32_t* d_c, uint32_t n0, uint32_t n1,
                         cudaStream_t st);
     void ensure_host_path();
+    uint32_t* staging(uint32_t*& h);
     void set_chunks(int want);
     template <class T>
     T* dalloc(size_t count);
@@ -133,6 +134,7 @@ private:
     uint32_t* ha_ = nullptr;  // pinned staging
     uint32_t* hb_ = nullptr;
     uint32_t* hc_ = nullptr;
+    uint32_t* herr_ = nullptr;   // pinned copy of the error word
     cudaStream_t stream_ = nullptr;   // kernels
     cudaStream_t copy_ = nullptr;     // host -> device
     cudaStream_t out_ = nullptr;      // device -> host
