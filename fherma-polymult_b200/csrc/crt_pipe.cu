@@ -121,9 +121,14 @@ __host__ __device__ inline uint32_t resident_b_bytes(int K, uint32_t U) {
     return static_cast<uint32_t>(nch - 1) * U * 128 + last_steps * 2 * U * 16;
 }
 
-Layout make_layout(int K, uint32_t U) {
+// cta_tiles: tiles a CTA takes; no ring is longer than its chunks (shared
+// memory that is not asked for lets the next kernel's blocks start beside this
+// one's).
+Layout make_layout(int K, uint32_t U, uint32_t cta_tiles) {
     Layout l{resident_b_bytes(K, U), kMaxSlots};
     while (l.slots > 2 && l.bytes() > kSmemLimit) --l.slots;
+    const uint32_t chunks = cta_tiles * ((static_cast<uint32_t>(K) + 1 + kChunk - 1) / kChunk);
+    if (l.slots > 2 * chunks) l.slots = 2 * chunks;
     return l;
 }
 
@@ -736,7 +741,7 @@ bool crt_pipe_supported(const DevPoint& d, const CrtConsts& cc, const uint32_t* 
     // coordinates (n_begin) a multiple of 4 words; the constants resident.
     return d.L >= 2 && d.crt_u <= 256 && d.K + 1 <= kMaxK && d.crt_img_v && (d.N & 3) == 0 && d.N >= kCrtTile &&
            (n_begin & 3) == 0 && n_end <= d.N && (reinterpret_cast<uintptr_t>(Y) & 15) == 0 &&
-           make_layout(d.K, d.crt_u).bytes() <= kSmemLimit && cc.est_err < 0.25f;
+           make_layout(d.K, d.crt_u, 1).bytes() <= kSmemLimit && cc.est_err < 0.25f;
 }
 
 void crt_pipe_init_attributes() {
@@ -750,7 +755,7 @@ void launch_crt_pipe(const DevPoint& d, const CrtConsts& cc, const uint32_t* Y, 
     if (n_end <= n_begin) return;
     const uint32_t tiles = (n_end - n_begin + kCrtTile - 1) / kCrtTile;
     const uint32_t grid = tiles < static_cast<uint32_t>(sms) ? tiles : static_cast<uint32_t>(sms);
-    const Layout lay = make_layout(d.K, d.crt_u);
+    const Layout lay = make_layout(d.K, d.crt_u, (tiles + grid - 1) / grid);
     // y: K rows of N words, boxes of 32 primes x 128 coefficients.
     const CUtensorMap tm = make_tmap_u32(Y, static_cast<uint64_t>(d.K), d.N, d.N, kChunk, kCrtTile, TmaSwizzle::kNone);
     const size_t smem = lay.bytes();

@@ -88,7 +88,9 @@ __host__ inline size_t smem_bytes(uint32_t kb, int nch, uint32_t cols, int L, Ri
 // K = 36, N = 2^17); L = 64 has room for two.  Other rows wait in the raw ring, four
 // tiles or more of it before a third operand slot.  Without room for a raw tile
 // they are copied word by word.
-__host__ inline Rings ring_sizes(uint32_t kb, int nch, uint32_t cols, int L) {
+// No ring is longer than the tiles a CTA takes: shared memory that is not
+// asked for is there for the next kernel's blocks.
+__host__ inline Rings ring_sizes(uint32_t kb, int nch, uint32_t cols, int L, uint32_t cta_tiles) {
     Rings r{2, 0};
     if (L & 3) {
         r = Rings{4, kMaxRaw};
@@ -99,6 +101,8 @@ __host__ inline Rings ring_sizes(uint32_t kb, int nch, uint32_t cols, int L) {
         r.slots = kMaxSlots;
         while (r.slots > 2 && smem_bytes(kb, nch, cols, L, r) > kSmemLimit) --r.slots;
     }
+    r.slots = r.slots < cta_tiles ? r.slots : cta_tiles;
+    r.raw = r.raw < cta_tiles ? r.raw : cta_tiles;
     return r;
 }
 
@@ -570,7 +574,7 @@ void launch_decompose_pipe(const DevPoint& d, const DecConsts& dc, const uint32_
     const uint32_t split = operands == 2 ? per : grid;
     const int nch = static_cast<int>(dc.chunks);
     const uint32_t cols = 16 * dc.piece;
-    const Rings rings = ring_sizes(d.dec_kb, nch, cols, d.L);
+    const Rings rings = ring_sizes(d.dec_kb, nch, cols, d.L, (tiles + per - 1) / per);
     const DecKernel kernel =
         rings.raw ? (dc.lazy_out ? dec_kernel<true, true>(dc.piece) : dec_kernel<false, true>(dc.piece))
                   : (dc.lazy_out ? dec_kernel<true, false>(dc.piece) : dec_kernel<false, false>(dc.piece));

@@ -64,7 +64,7 @@ void build_row_tables(const DevPoint& d, uint2* out, cudaStream_t st);
 // prime (products whose clusters are all resident at once).  N = 2^8 .. 2^10 read tables of their own, K x N pairs from
 // build_whole_tables (DevPoint::row_tw).
 bool ntt_fused_ok(const DevPoint& d, int mode, int sms);
-void launch_ntt_fused(const DevPoint& d, uint32_t* A, uint32_t* B, int mode, cudaStream_t st);
+void launch_ntt_fused(const DevPoint& d, uint32_t* A, uint32_t* B, int mode, int sms, cudaStream_t st);
 void build_whole_tables(const DevPoint& d, uint2* out, cudaStream_t st);
 void ntt_fused_init_attributes();
 

@@ -1073,7 +1073,7 @@ void launch_ntt(const DevPoint& d, uint32_t* A, uint32_t* B, int mode, cudaStrea
     // the separate passes where there are any.
     const int m = d.logR == 0 && mode == kPassRow ? static_cast<int>(kRowProduct) : mode;
     if (ntt_fused_ok(d, m, device_sms()) && (d.logR == 0 || col_pass_variant() == 0)) {
-        launch_ntt_fused(d, A, B, m, st);
+        launch_ntt_fused(d, A, B, m, device_sms(), st);
         return;
     }
     if (d.logN <= kSmallLogN) {

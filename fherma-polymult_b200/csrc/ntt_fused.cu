@@ -27,6 +27,7 @@
 #include "pdl.cuh"
 #include "tc.cuh"
 
+#include <algorithm>
 #include <stdexcept>
 
 namespace fpm {
@@ -121,8 +122,10 @@ __global__ void __launch_bounds__(ClusterGeom<LOGS>::T, ClusterGeom<LOGS>::kBloc
     const SharedTable fcol{cf}, icol{ci};
     const RowTable<LOGS, RG::kStride, false, RG::kFlip> fw{tf};
     const RowTable<LOGS, RG::kStride, true, RG::kFlip> iw{tf};
-    pdl_launch_dependents();
+    // (The CRT's blocks may start once these are at work: let in before the
+    // wait they took their places, N = 4096 K = 19 13.4 us a product for 11.1.)
     pdl_wait();
+    pdl_launch_dependents();
 
     // Forward column pass; the last round's results go to the row tiles.
     {
@@ -329,11 +332,19 @@ __global__ void __launch_bounds__(256) k_whole_tables(DevPoint d, int rb, uint2*
 }
 
 template <bool LAZY>
-void launch_cluster(const DevPoint& d, uint32_t* A, uint32_t* B, cudaStream_t st) {
+void launch_cluster(const DevPoint& d, uint32_t* A, uint32_t* B, int sms, cudaStream_t st) {
     auto run = [&](auto ls) {
         using CG = ClusterGeom<decltype(ls)::value>;
-        check(launch_pdl_cluster(k_ntt_cluster<decltype(ls)::value, LAZY>, dim3(CG::kCtas, d.K), dim3(CG::T), CG::kCtas,
-                                 CG::kSmem, st, d, A, B),
+        // Started under the decompose's tail, clusters crowd onto the SMs it
+        // leaves free and stay there: only if those take them one by one
+        // (the decompose runs a CTA per 128 coefficients and operand, up to one
+        // an SM).  Product us, early | not: N = 4096 K = 19 11.1 | 12.4, K = 60
+        // 19.6 | 16.8, N = 8192 K = 10 17.6 | 14.7, K = 139 32.0 | 29.5, N = 16384
+        // K = 10 19.4 | 15.8, K = 36 22.4 | 21.1.
+        const uint32_t busy = std::min<uint32_t>(sms, d.N / 64);
+        const bool early = CG::kCtas * static_cast<uint32_t>(d.K) <= static_cast<uint32_t>(sms) - busy;
+        check(launch_cluster_grid(k_ntt_cluster<decltype(ls)::value, LAZY>, dim3(CG::kCtas, d.K), dim3(CG::T), CG::kCtas,
+                                  early, CG::kSmem, st, d, A, B),
               "transform launch");
     };
     switch (d.logS) {
@@ -405,11 +416,11 @@ bool ntt_fused_ok(const DevPoint& d, int mode, int sms) {
     return ctas <= ClusterGeom<6>::kBlocks * sms;
 }
 
-void launch_ntt_fused(const DevPoint& d, uint32_t* A, uint32_t* B, int mode, cudaStream_t st) {
+void launch_ntt_fused(const DevPoint& d, uint32_t* A, uint32_t* B, int mode, int sms, cudaStream_t st) {
     if (d.logN <= 11) {
         d.lazy ? launch_whole<true>(d, A, B, mode, st) : launch_whole<false>(d, A, B, mode, st);
     } else {
-        d.lazy ? launch_cluster<true>(d, A, B, st) : launch_cluster<false>(d, A, B, st);
+        d.lazy ? launch_cluster<true>(d, A, B, sms, st) : launch_cluster<false>(d, A, B, sms, st);
     }
 }
 

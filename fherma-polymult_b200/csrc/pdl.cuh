@@ -36,10 +36,11 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-// The same with the grid's blocks in clusters of `ctas` along x.
+// A grid of clusters of `ctas` blocks along x, with (early) or without that
+// attribute.
 template <class... KArgs, class... Args>
-cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, uint32_t ctas, size_t smem,
-                               cudaStream_t st, Args&&... args) {
+cudaError_t launch_cluster_grid(void (*kernel)(KArgs...), dim3 grid, dim3 block, uint32_t ctas, bool early, size_t smem,
+                                cudaStream_t st, Args&&... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -47,7 +48,7 @@ cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, 
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = ctas;
     attr[1].val.clusterDim.y = 1;
