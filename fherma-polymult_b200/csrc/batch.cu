@@ -48,6 +48,11 @@ struct TransformClass {
     }
 };
 
+// Branches that whole one-product chains are spread over (layout 2).  Three: 16
+// products of the benchmark mix took 584 us on two, 595 on three, 628 on four;
+// 8 took 332, 299, 312 (B200, as plain calls on that many streams of a graph).
+constexpr size_t kChainBranches = 3;
+
 }  // namespace
 
 uint64_t occupancy_key(int pass, uint32_t logR, uint32_t logS, bool lazy) {
@@ -292,15 +297,49 @@ int enqueue_grouped(const std::vector<GroupedProduct>& prods_, const BatchSchedu
         small_ntt(small, st);
         crt(all, st);
     } else {
-        size_t b = 0;
+        // The products with pipelines of their own run as a plain call does,
+        // chain by chain (each one's residues stay in L2 from launch to launch),
+        // spread over the branches by cost, largest first; the rest as one
+        // grouped chain per geometry, on a branch each.
         std::vector<cudaStream_t> used;
+        std::vector<double> load;
+        auto take = [&](size_t k) {
+            while (used.size() <= k) {
+                cudaStream_t s = env.branches.at(used.size());
+                fork(st, s);
+                used.push_back(s);
+                load.push_back(0);
+            }
+            return used[k];
+        };
+        std::vector<size_t> alone;
+        size_t k = 0;
         for (auto& kv : classes) {
-            cudaStream_t s = env.branches.at(b++);
-            fork(st, s);
-            decompose(kv.second, s);
-            transform(kv.first, kv.second, s);
-            crt(kv.second, s);
-            used.push_back(s);
+            std::vector<size_t> rest;
+            double cost = 0;
+            for (size_t i : kv.second) {
+                if (piped(prods_[i])) {
+                    alone.push_back(i);
+                } else {
+                    rest.push_back(i);
+                    cost += prods_[i].cost;
+                }
+            }
+            if (rest.empty()) continue;
+            cudaStream_t s = take(k);
+            decompose(rest, s);
+            transform(kv.first, rest, s);
+            crt(rest, s);
+            load[k++] += cost;
+        }
+        std::stable_sort(alone.begin(), alone.end(),
+                         [&](size_t x, size_t y) { return prods_[x].cost > prods_[y].cost; });
+        if (!alone.empty()) take(std::min(alone.size(), kChainBranches) - 1);
+        for (size_t i : alone) {
+            const size_t to = std::min_element(load.begin(), load.end()) - load.begin();
+            const GroupedProduct& p = prods_[i];
+            launches_ += p.e->product_on(p.d, p.a, p.b, p.A, p.B, p.c, used[to]);
+            load[to] += p.cost;
         }
         decompose(small, st);
         small_ntt(small, st);
@@ -440,7 +479,7 @@ void Batch::build_graph() {
             if (!occupancy_.count(k)) occupancy_[k] = ntt_mixed_occupancy(pass, lz == 1, max_log_s[lz]);
         }
     }
-    for (size_t i = 0; i < classes; ++i) branch(i);
+    for (size_t i = 0; i < std::max(classes, kChainBranches); ++i) branch(i);
     exec_ = capture(prods_, &launches_);
 }
 
@@ -543,7 +582,7 @@ double Batch::tune(int reps) {
     for (int layout : {0, 1, 2, 3})
         for (int grp : {0, 16})
             for (int grid : {0, 1})
-                for (int pipe : {0, 14, 16}) cands.push_back(BatchSchedule{layout, 1, grp, grid, pipe});
+                for (int pipe : {0, 12, 14}) cands.push_back(BatchSchedule{layout, 1, grp, grid, pipe});
     cudaEvent_t t0 = nullptr, t1 = nullptr;
     check(cudaEventCreate(&t0), "event");
     check(cudaEventCreate(&t1), "event");

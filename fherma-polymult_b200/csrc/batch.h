@@ -28,7 +28,8 @@ namespace fpm {
 
 struct BatchSchedule {
     int layout = 1;        // 0 one stream; 1 geometry chains as branches between the shared
-                           // decompose and CRT; 2 a whole branch (decompose .. CRT) per geometry;
+                           // decompose and CRT; 2 a whole branch (decompose .. CRT) per geometry,
+                           // products at or above pipe_min_log_n as chains of their own;
                            // 3 one launch per stage: each transform pass covers every R = 64
                            // product whatever its row length (mixed-geometry kernels)
     int order = 1;         // 0 products as given; 1 largest first

@@ -274,7 +274,7 @@ void Engine::launch_dec(const uint32_t* d_limbs, uint32_t* d_res, int operand, u
 }
 
 void Engine::launch_crt_any(const DevPoint& d, const uint32_t* d_y, uint32_t* d_c, uint32_t n0, uint32_t n1,
-                            cudaStream_t st) {
+                            cudaStream_t st) const {
     if (simt_ || !crt_uses_tc(plan_)) {
         launch_crt(d, d_y, d_c, n0, n1, st);
     } else if (crt_consts_ && crt_pipe_supported(d, *crt_consts_, d_y, n0, n1)) {
@@ -309,7 +309,7 @@ void Engine::transform(uint32_t* d_A, uint32_t* d_B, int mode, cudaStream_t st) 
 // Both operands' decompose, as a product launches it (one paired launch on the
 // tensor-core paths).
 void Engine::decompose_pair_on(const DevPoint& d, const uint32_t* a, const uint32_t* b, uint32_t* A, uint32_t* B,
-                               cudaStream_t st) {
+                               cudaStream_t st) const {
     if (simt_) {
         launch_decompose(d, a, A, 0, 0, plan_.N, st);
         launch_decompose(d, b, B, 1, 0, plan_.N, st);
@@ -331,17 +331,18 @@ void Engine::crt(const uint32_t* d_y, uint32_t* d_c, cudaStream_t st) {
     check(cudaGetLastError(), "crt launch");
 }
 
-void Engine::product(const DevPoint& d, const uint32_t* d_a, const uint32_t* d_b, uint32_t* A, uint32_t* B,
-                     uint32_t* d_c, cudaStream_t st) {
+int Engine::product_on(const DevPoint& d, const uint32_t* d_a, const uint32_t* d_b, uint32_t* A, uint32_t* B,
+                       uint32_t* d_c, cudaStream_t st) const {
     const uint32_t N = plan_.N;
     decompose_pair_on(d, d_a, d_b, A, B, st);
     launch_ntt(d, A, B, kRowProduct, st);
     launch_crt_any(d, A, d_c, 0, N, st);
     check(cudaGetLastError(), "product launch");
+    return (simt_ ? 2 : 1) + ntt_launches(d) + 1;
 }
 
 void Engine::run_device(const uint32_t* d_a, const uint32_t* d_b, uint32_t* d_c, cudaStream_t st) {
-    product(dp_, d_a, d_b, A_, B_, d_c, st);
+    product_on(dp_, d_a, d_b, A_, B_, d_c, st);
 }
 
 namespace {
@@ -474,7 +475,7 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c, uint32_
     const bool small = nch == 1 && all <= (size_t(256) << 10);
     if (small) {
         for (int op = 0; op < 2; ++op) bring_in(op, 0, all, stream_);
-        product(dp_, la_, lb_, A_, B_, lc_, stream_);
+        product_on(dp_, la_, lb_, A_, B_, lc_, stream_);
         check(cudaMemcpyAsync(dst, lc_, all, cudaMemcpyDeviceToHost, stream_), "copy out");
         check(cudaMemcpyAsync(herr_, dp_.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream_), "read error word");
         check(cudaEventRecord(out_ev[0], stream_), "event");

@@ -93,22 +93,23 @@ public:
     // ((K + 1) x L), to host memory; returns K.
     uint32_t crt_tables(uint32_t* M, uint32_t* negvP) const;
 
+    // One product on workspaces A, B with point d (whose err names the error
+    // word to use), enqueued on st; returns its number of launches.
+    int product_on(const DevPoint& d, const uint32_t* d_a, const uint32_t* d_b, uint32_t* A, uint32_t* B, uint32_t* d_c,
+                   cudaStream_t st) const;
+
     size_t words() const { return static_cast<size_t>(plan_.N) * plan_.L; }
     size_t residues() const { return static_cast<size_t>(plan_.K) * plan_.N; }
 
 private:
     size_t static_scratch_err_offset() const;
-    // The product's launches on workspaces A, B with point d (whose err names
-    // the error word to use).
-    void product(const DevPoint& d, const uint32_t* d_a, const uint32_t* d_b, uint32_t* A, uint32_t* B, uint32_t* d_c,
-                 cudaStream_t st);
     void release();
     void decompose_pair_on(const DevPoint& d, const uint32_t* a, const uint32_t* b, uint32_t* A, uint32_t* B,
-                           cudaStream_t st);
+                           cudaStream_t st) const;
     void launch_dec(const uint32_t* d_limbs, uint32_t* d_res, int operand, uint32_t n0, uint32_t n1,
                     cudaStream_t st);
     void launch_crt_any(const DevPoint& d, const uint32_t* d_y, uint32_t* d_c, uint32_t n0, uint32_t n1,
-                        cudaStream_t st);
+                        cudaStream_t st) const;
     void ensure_host_path();
     uint32_t* staging(uint32_t*& h);
     void set_chunks(int want);

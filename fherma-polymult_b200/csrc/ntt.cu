@@ -1090,6 +1090,12 @@ void launch_ntt(const DevPoint& d, uint32_t* A, uint32_t* B, int mode, cudaStrea
     }
 }
 
+int ntt_launches(const DevPoint& d) {
+    const bool one = d.logN <= kSmallLogN || (ntt_fused_ok(d, kRowProduct, device_sms()) &&
+                                              (d.logR == 0 || col_pass_variant() == 0));
+    return one ? 1 : 3;
+}
+
 uint32_t ntt_blocks_per_prime(int pass, uint32_t logR, uint32_t logS) {
     if (pass == kPassRow) {
         const uint32_t G = 2048u >> logS;

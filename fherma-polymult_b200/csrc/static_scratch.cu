@@ -92,7 +92,7 @@ void Engine::run_device_static(const uint32_t* d_a, const uint32_t* d_b, uint32_
     uint32_t* base = static_cast<uint32_t*>(scratch_address(cur));
     DevPoint d = dp_;
     d.err = base + static_scratch_err_offset();
-    product(d, d_a, d_b, base, base + residues(), d_c, st);
+    product_on(d, d_a, d_b, base, base + residues(), d_c, st);
 }
 
 uint32_t Engine::take_static_error(cudaStream_t st) {

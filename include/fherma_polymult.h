@@ -191,7 +191,9 @@ typedef struct fpm_batch fpm_batch;
 typedef struct fpm_batch_info {
     uint32_t count;        /* products */
     int32_t layout;        /* 0 one stream; 1 transform geometries as parallel graph
-                              branches; 2 a whole branch per geometry; 3 one launch per
+                              branches; 2 a whole branch per geometry, products at or
+                              above pipe_min_log_n as chains of their own over three
+                              branches; 3 one launch per
                               stage (every transform pass covers all products with
                               N = 2^12 .. 2^17 in one launch, whatever their lengths) */
     int32_t order;         /* 0 as given; 1 largest product first */
