@@ -12,14 +12,10 @@
 // top limb and the rounding sum run on the CUDA cores.  The prime basis covers
 // 2^20 N q^2, so sum_j y_j / p_j lies within 2^-21 of an integer v and any
 // estimate within 1/2 - 2^-21 rounds to it.  The stagers sum in single
-// precision: x = y_j >> sh_j (sh_j = bits of p_j - 23, so x < 2^23) is formed
-// exactly as the float 2^23 + x by setting the exponent bits, multiplied by
-// cf_j = 2^sh_j / p_j and added with FFMA; the 2^23 cf_j parts (each at most
-// 2) add up to the constant voff, removed at the end.  Error: the dropped low
-// bits, below 2^sh_j / p_j <= 2^-22 per term, and the roundings, below 2^-24
-// of partial sums under 3 (K + 1) each; the host bounds the total
-// (CrtConsts::est_err, 2^-8 at K = 160) and the kernel is used only while it
-// is under 1/4.
+// precision, y_j rounded to a float times 1 / p_j by FFMA: each term is off by
+// less than 2^-23 and each of the roundings of a partial sum by less than
+// 2^-24 (K + 1); the host bounds the total (CrtConsts::est_err, 2^-9 at K = 160)
+// and the kernel is used only while it is under 1/4.
 //
 // Organisation on the B200: one CTA per SM walks tiles of 128 coefficients
 // (one MMA M); tile i of a CTA accumulates into TMEM buffer i % 2 (256 columns
@@ -89,9 +85,9 @@ constexpr uint32_t kMaxASlots = 2;
 // are boxes, the last na operands.
 constexpr uint32_t kSlot = kChunk * kCrtTile * 4;
 constexpr size_t kSmemLimit = 227 * 1024;
-// Shared copies of the constants: {cf_j bits, top_j, sh_j, 0} per row
-// j < 32 nch (zero beyond the K + 1 rows), then q.
-constexpr size_t kConstBytes = (kMaxK + 1) * sizeof(uint4) + ((kMaxL + 2) * 4 + 15) / 16 * 16;
+// Shared copies of the constants: {1 / p_j bits, top_j} per row j < 32 nch
+// (zero beyond the K + 1 rows; kMaxK + 2 entries, a multiple of 16 bytes), then q.
+constexpr size_t kConstBytes = (kMaxK + 2) * sizeof(uint2) + ((kMaxL + 2) * 4 + 15) / 16 * 16;
 
 constexpr int kBars = 34;
 
@@ -138,7 +134,7 @@ struct Smem {
     uint8_t* aop;        // [na][kSlot] A operands
     uint4* meta;         // [2][128] {top-limb words 0, 1, 2, -}
     uint4* xch;          // [2][128] second halves' sums {rounding sum, top-limb words 0, 1, 2}
-    uint4* kc;           // [kMaxK + 1] {cf_j bits, top_j, sh_j, 0}
+    uint2* kc;           // [kMaxK + 2] {1 / p_j bits, top_j}
     uint32_t* qs;        // [L + 2] q, zero above L
     uint64_t* b_full;    // [1] the constant image landed
     uint64_t* y_full;    // [kMaxSlots] the slot's TMA box landed
@@ -161,8 +157,8 @@ __device__ inline Smem carve(uint8_t* base, const Layout& lay) {
     s.aop = s.slot + lay.ny() * kSlot;
     s.meta = reinterpret_cast<uint4*>(base + lay.meta_off());
     s.xch = reinterpret_cast<uint4*>(base + lay.xch_off());
-    s.kc = reinterpret_cast<uint4*>(base + lay.const_off());
-    s.qs = reinterpret_cast<uint32_t*>(base + lay.const_off() + (kMaxK + 1) * sizeof(uint4));
+    s.kc = reinterpret_cast<uint2*>(base + lay.const_off());
+    s.qs = reinterpret_cast<uint32_t*>(base + lay.const_off() + (kMaxK + 2) * sizeof(uint2));
     uint64_t* bars = reinterpret_cast<uint64_t*>(base + lay.bar_off());
     s.b_full = bars;
     s.y_full = bars + 1;
@@ -351,7 +347,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
     }
     for (int j = threadIdx.x; j <= kMaxK; j += kThreads)
-        sm.kc[j] = make_uint4(j < K ? __float_as_uint(cc.cf[j]) : 0u, j <= K ? cc.top[j] : 0u, j < K ? cc.sh[j] : 0u, 0u);
+        sm.kc[j] = make_uint2(j < K ? __float_as_uint(cc.cf[j]) : 0u, j <= K ? cc.top[j] : 0u);
     for (int k = threadIdx.x; k < kMaxL + 2; k += kThreads) sm.qs[k] = cc.q[k];
     if (warp == kYWarp && lane == 0) tc::prefetch_tmap(&tmY);
     if (warp == 0) tc::tmem_alloc(sm.tmem_base, 512);
@@ -459,19 +455,16 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const uint32_t yrow = tc::smem_addr(sm.slot + ys * kSlot) + 4 * (h * kHalf * kCrtTile + m);
 #pragma unroll
                 for (int jj = 0; jj < kHalf; ++jj) yv[jj] = tc::ld_shared_once(yrow + 4 * jj * kCrtTile);
-                // Rows j >= K of the box read as zero and cf_j = 0 there, so
-                // every row of the chunk takes part without a test.
-                const uint4* kc = sm.kc + c * static_cast<int>(kChunk) + h * kHalf;
+                // Rows j >= K of the box read as zero and 1 / p_j as 0, so every
+                // row of the chunk takes part without a test.
+                const uint4* kc = reinterpret_cast<const uint4*>(sm.kc + c * static_cast<int>(kChunk) + h * kHalf);
 #pragma unroll
                 for (int q2 = 0; q2 < kHalf / 2; ++q2) {
-                    uint64_t grp = 0;
-#pragma unroll
-                    for (int jj = 2 * q2; jj < 2 * q2 + 2; ++jj) {
-                        const uint4 kj = kc[jj];
-                        const float yf = __uint_as_float((yv[jj] >> kj.z) + 0x4B000000u);
-                        vf[jj % kPart] = fmaf(yf, __uint_as_float(kj.x), vf[jj % kPart]);
-                        grp += static_cast<uint64_t>(yv[jj]) * kj.y;
-                    }
+                    const uint4 kj = kc[q2];   // two primes
+                    const uint32_t y0 = yv[2 * q2], y1 = yv[2 * q2 + 1];
+                    vf[(2 * q2) % kPart] = fmaf(__uint2float_rn(y0), __uint_as_float(kj.x), vf[(2 * q2) % kPart]);
+                    vf[(2 * q2 + 1) % kPart] = fmaf(__uint2float_rn(y1), __uint_as_float(kj.z), vf[(2 * q2 + 1) % kPart]);
+                    const uint64_t grp = static_cast<uint64_t>(y0) * kj.y + static_cast<uint64_t>(y1) * kj.w;
                     t01 += grp;
                     t2 += t01 < grp ? 1u : 0u;
                 }
@@ -500,7 +493,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     if (!ok) break;
                     const float vh = (vf[0] + vf[1]) + (vf[2] + vf[3]);
                     const uint4 x = sm.xch[xb * kCrtTile + m];
-                    int v = __float2int_rn((vh + __uint_as_float(x.x)) - cc.voff);
+                    int v = __float2int_rn(vh + __uint_as_float(x.x));
                     v = v < 0 ? 0 : (v > K ? K : v);
                     const uint32_t vu = live ? static_cast<uint32_t>(v) : 0u;
                     const uint64_t other = (static_cast<uint64_t>(x.z) << 32) | x.y;
@@ -710,27 +703,15 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 CrtConsts make_crt_consts(const HostPlan& pl, const uint32_t* top) {
     CrtConsts cc{};
-    // The rounding sum's constants and its error bound (see the head of
-    // this file): truncation sum_j 2^sh_j / p_j, one rounding of a partial
-    // sum per term, the final adds and voff's own rounding.
-    double off = 0, trunc = 0, tmax = 0;
+    // The rounding sum's constants and a bound on its error (see the head of
+    // this file): per term y_j's and 1 / p_j's roundings (y_j / p_j < 1), and one
+    // rounding of a sum below K + 1 per term and per final addition.
     for (int j = 0; j <= pl.K; ++j) {
-        if (j < pl.K) {
-            const uint32_t p = pl.primes[j];
-            int bits = 0;
-            while (bits < 32 && (p >> bits) != 0) ++bits;
-            const uint32_t sh = bits > 23 ? static_cast<uint32_t>(bits - 23) : 0u;
-            cc.sh[j] = sh;
-            cc.cf[j] = static_cast<float>(std::ldexp(1.0, static_cast<int>(sh)) / p);
-            off += 8388608.0 * static_cast<double>(cc.cf[j]);
-            trunc += std::ldexp(1.0, static_cast<int>(sh)) / p;
-            tmax += 2 * 8388608.0 * static_cast<double>(cc.cf[j]);
-        }
+        if (j < pl.K) cc.cf[j] = static_cast<float>(1.0 / pl.primes[j]);
         cc.top[j] = top[j];
     }
-    cc.voff = static_cast<float>(off);
     const double ulp = std::ldexp(1.0, -24);
-    cc.est_err = static_cast<float>(trunc + (pl.K + 4) * tmax * ulp + off * ulp);
+    cc.est_err = static_cast<float>(3 * pl.K * ulp + (pl.K + 8.0) * (pl.K + 1.0) * ulp);
     for (int k = 0; k < pl.L; ++k) cc.q[k] = pl.q[k];
     return cc;
 }

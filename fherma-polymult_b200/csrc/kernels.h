@@ -87,9 +87,7 @@ void launch_crt_tc(const DevPoint& d, const uint32_t* Y, uint32_t* c, uint32_t n
 // Needs L >= 2 and N, n_begin, n_end multiples of 4.  Its per-prime constants
 // travel as a kernel parameter.
 struct CrtConsts {
-    float cf[kMaxK];            // 2^sh_j / p_j in single precision, for the rounding sum
-    uint32_t sh[kMaxK];         // sh_j: y_j >> sh_j < 2^23 and 2^(23 + sh_j) / p_j <= 2
-    float voff;                 // sum_j 2^23 cf_j: the offset the rounding sum removes
+    float cf[kMaxK];            // 1 / p_j in single precision, for the rounding sum
     float est_err;              // a bound on the rounding sum's error (must stay below 1/4)
     uint32_t top[kMaxK + 1];    // top limb of constant j (j = K: -P mod q)
     uint32_t q[kMaxL + 2];      // q, zero above L
