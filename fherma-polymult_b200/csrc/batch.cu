@@ -67,13 +67,13 @@ int enqueue_grouped(const std::vector<GroupedProduct>& prods_, const BatchSchedu
     if (sched_.order == 1) {
         std::stable_sort(ord.begin(), ord.end(), [&](size_t x, size_t y) { return prods_[x].cost > prods_[y].cost; });
     }
-    // Products by transform geometry; N <= 1024 runs the one-block-per-prime
-    // kernel, product by product.
+    // Products by transform geometry; N <= 2048 runs the one-block-per-prime
+    // kernels, product by product.
     std::map<TransformClass, std::vector<size_t>> classes;
     std::vector<size_t> small;
     for (size_t i : ord) {
         const DevPoint& d = prods_[i].d;
-        if (d.logN <= kSmallLogN) {
+        if (d.logR == 0) {
             small.push_back(i);
         } else {
             classes[TransformClass{d.logR, d.logS, d.lazy != 0}].push_back(i);
@@ -457,7 +457,7 @@ void Batch::build_graph() {
     size_t classes = 0;
     std::vector<uint32_t> seen;
     for (const GroupedProduct& p : prods_) {
-        if (p.d.logN <= kSmallLogN) continue;
+        if (p.d.logR == 0) continue;
         const uint32_t key = p.d.logR * 64 + p.d.logS * 2 + (p.d.lazy ? 1 : 0);
         if (std::find(seen.begin(), seen.end(), key) != seen.end()) continue;
         seen.push_back(key);

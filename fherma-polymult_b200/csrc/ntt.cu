@@ -305,10 +305,9 @@ __global__ void __launch_bounds__(256, 8) k_ntt_col_inv_tma(DevPoint d, const __
 }
 
 // ---------------------------------------------------------------------------
-// Row pass.  A block owns G = 2048 / S rows of one prime: tile row g < G/2 is
+// Row pass.  A block owns G rows of one prime (RowGeom): tile row g < G/2 is
 // row u0 + g, tile row g >= G/2 is row R - 1 - u0 - (g - G/2), so rows g and
-// g ^ G/2 are partners (u, R - 1 - u).  With G = 1 (S = 2048) the block owns one
-// row and builds its partner's table beside its own.
+// g ^ G/2 are partners (u, R - 1 - u).
 //
 // Forward table of row u, entry y in [2^lev, 2^(lev+1)), stage b = LOGS-1-lev:
 // psi^(2^b (1 + 2 bitrev(u)) + 2^(b+1+logR) bitrev(y - 2^lev)) = U[u][b] Q[y].
@@ -363,10 +362,15 @@ __device__ __forceinline__ size_t row_offset(uint32_t i, uint32_t u0, uint32_t R
     return static_cast<size_t>(row_of_slot<LOGS>(i >> LOGS, u0, R)) * (1u << LOGS) + (i & ((1u << LOGS) - 1u));
 }
 
+template <int LOGS>
+constexpr int row_threads() {
+    return 1 << (RowGeom<LOGS>::kBits - row_pass_rb(LOGS));
+}
+
 // The row pass's tables barrier sits after the tiles and the tables.
 template <int LOGS>
 constexpr size_t row_bar_offset() {
-    return 2 * 2048 * sizeof(uint32_t) + RowGeom<LOGS>::kSlots * RowGeom<LOGS>::kStride * sizeof(uint2);
+    return 2 * RowGeom<LOGS>::kTile * sizeof(uint32_t) + RowGeom<LOGS>::kSlots * RowGeom<LOGS>::kStride * sizeof(uint2);
 }
 
 // phase: parity of this tile's use of the tables barrier (the block's tile
@@ -377,13 +381,14 @@ template <int LOGS, bool LAZY, class TEAM = BlockTeam, bool PDL = false>
 __device__ __forceinline__ void row_body(const DevPoint& d, uint32_t* A, uint32_t* B, int mode, int j, uint32_t bx,
                                          uint32_t phase, uint32_t* smem, uint64_t* tbar) {
     using RG = RowGeom<LOGS>;
-    constexpr int RB = row_pass_rb(LOGS), E = 1 << RB, T = ntt_threads<RB>();
-    using RPR = RP<LOGS, 0, SwzRow, RB>;
+    constexpr int RB = row_pass_rb(LOGS), E = 1 << RB, T = row_threads<LOGS>();
+    using SWZ = RowSwz<LOGS>;
+    using RPR = RP<LOGS, 0, SWZ, RB>;
     static_assert(RPR::all_conflict_free(), "row rounds must be free of bank conflicts");
     constexpr int last = RPR::kCount - 1;
     uint32_t* ta = smem;
-    uint32_t* tb = smem + 2048;
-    uint2* tf = reinterpret_cast<uint2*>(smem + 4096);
+    uint32_t* tb = smem + RG::kTile;
+    uint2* tf = reinterpret_cast<uint2*>(smem + 2 * RG::kTile);
     const uint32_t u0 = bx * RG::kPairsPerBlock;
     const uint32_t R = 1u << d.logR;
     const PrimeConsts pc = d.pc[j];
@@ -400,7 +405,7 @@ __device__ __forceinline__ void row_body(const DevPoint& d, uint32_t* A, uint32_
     // Round 0 straight from global memory (the thread's E elements lie in one
     // row).
     {
-        const uint32_t base = round_base<LOGS, 0, SwzRow, RB, 0>(TEAM::tid());
+        const uint32_t base = round_base<LOGS, 0, SWZ, RB, 0>(TEAM::tid());
         constexpr int sh = RPR::lo(0);
         uint32_t v[2][E];
         const size_t at = row_offset<LOGS>(base, u0, R);
@@ -412,20 +417,20 @@ __device__ __forceinline__ void row_body(const DevPoint& d, uint32_t* A, uint32_
         // The bound only guards against a copy that never lands: past it the
         // error word gets bit 2 and the block goes on (with wrong twiddles).
         if (!tc::wait_parity(tbar, phase, d.wait_ns) && (TEAM::tid() & 31) == 0) atomicOr(d.err, 4u);
-        fwd_round<LOGS, 0, SwzRow, RB, 0, LAZY, 2>(v, base, fw, p);
+        fwd_round<LOGS, 0, SWZ, RB, 0, LAZY, 2>(v, base, fw, p);
 #pragma unroll
-        for (int o = 0; o < 2; ++o) store_round<LOGS, 0, SwzRow, RB, 0>(tiles[o], v[o], base);
+        for (int o = 0; o < 2; ++o) store_round<LOGS, 0, SWZ, RB, 0>(tiles[o], v[o], base);
         TEAM::sync();
     }
-    fwd_range<LOGS, 0, SwzRow, RB, 1, last, LAZY, 2, TEAM>(tiles, fw, p);
+    fwd_range<LOGS, 0, SWZ, RB, 1, last, LAZY, 2, TEAM>(tiles, fw, p);
     // Last forward round, the pointwise product and the first inverse round in
     // registers.
     {
-        const uint32_t base = round_base<LOGS, 0, SwzRow, RB, last>(TEAM::tid());
+        const uint32_t base = round_base<LOGS, 0, SWZ, RB, last>(TEAM::tid());
         uint32_t v[2][E];
-        load_round<LOGS, 0, SwzRow, RB, last>(ta, v[0], base);
-        load_round<LOGS, 0, SwzRow, RB, last>(tb, v[1], base);
-        fwd_round<LOGS, 0, SwzRow, RB, last, LAZY, 2>(v, base, fw, p);
+        load_round<LOGS, 0, SWZ, RB, last>(ta, v[0], base);
+        load_round<LOGS, 0, SWZ, RB, last>(tb, v[1], base);
+        fwd_round<LOGS, 0, SWZ, RB, last, LAZY, 2>(v, base, fw, p);
         if (mode == kRowForward) {
             if constexpr (LAZY) {
 #pragma unroll
@@ -434,35 +439,30 @@ __device__ __forceinline__ void row_body(const DevPoint& d, uint32_t* A, uint32_
                     v[1][k] = canon4(v[1][k], p);
                 }
             }
-            store_round<LOGS, 0, SwzRow, RB, last>(ta, v[0], base);
-            store_round<LOGS, 0, SwzRow, RB, last>(tb, v[1], base);
+            store_round<LOGS, 0, SWZ, RB, last>(ta, v[0], base);
+            store_round<LOGS, 0, SWZ, RB, last>(tb, v[1], base);
             TEAM::sync();
-            for (uint32_t i = TEAM::tid(); i < 2048; i += T) {
+            for (uint32_t i = TEAM::tid(); i < RG::kTile; i += T) {
                 const size_t at = row_offset<LOGS>(i, u0, R);
-                a[at] = ta[SwzRow::f(i)];
-                b[at] = tb[SwzRow::f(i)];
+                a[at] = ta[SWZ::f(i)];
+                b[at] = tb[SWZ::f(i)];
             }
             return;
         }
 #pragma unroll
         for (int k = 0; k < E; ++k) v[0][k] = pointwise<LAZY>(v[0][k], v[1][k], pc);
-        inv_round<LOGS, 0, SwzRow, RB, last, LAZY, true>(v[0], base, iw, p);
-        store_round<LOGS, 0, SwzRow, RB, last>(ta, v[0], base);
+        inv_round<LOGS, 0, SWZ, RB, last, LAZY, true>(v[0], base, iw, p);
+        store_round<LOGS, 0, SWZ, RB, last>(ta, v[0], base);
         TEAM::sync();
     }
-    inv_range<LOGS, 0, SwzRow, RB, last - 1, 1, LAZY, true, TEAM>(ta, iw, p);
+    inv_range<LOGS, 0, SWZ, RB, last - 1, 1, LAZY, true, TEAM>(ta, iw, p);
     // Inverse round 0 straight to global memory.
     {
-        const uint32_t base = round_base<LOGS, 0, SwzRow, RB, 0>(TEAM::tid());
+        const uint32_t base = round_base<LOGS, 0, SWZ, RB, 0>(TEAM::tid());
         constexpr int sh = RPR::lo(0);
         uint32_t v[E];
-        load_round<LOGS, 0, SwzRow, RB, 0>(ta, v, base);
-        inv_round<LOGS, 0, SwzRow, RB, 0, LAZY, true>(v, base, iw, p);
-        if (LAZY && d.logR == 0) {
-            // No column pass follows: these are the y_j, canonical for the CRT.
-#pragma unroll
-            for (int k = 0; k < E; ++k) v[k] = reduce_once(v[k], p);
-        }
+        load_round<LOGS, 0, SWZ, RB, 0>(ta, v, base);
+        inv_round<LOGS, 0, SWZ, RB, 0, LAZY, true>(v, base, iw, p);
         const size_t at = row_offset<LOGS>(base, u0, R);
 #pragma unroll
         for (int k = 0; k < E; ++k) a[at + (k << sh)] = v[k];
@@ -477,10 +477,6 @@ template <int LOGR>
 constexpr int col_threads() {
     return ntt_threads<col_pass_rb(LOGR)>();
 }
-template <int LOGS>
-constexpr int row_threads() {
-    return ntt_threads<row_pass_rb(LOGS)>();
-}
 template <int LOGR, int MIN8>
 constexpr int col_min_blocks() {
     return col_pass_rb(LOGR) == 3 ? MIN8 : 8;
@@ -489,9 +485,10 @@ constexpr int col_min_blocks() {
 // five of 128 (16-element rounds, up to 96 registers).  At N = 65536 (K = 139)
 // the 16-element row pass measured 54.9 us with five blocks per SM against
 // 56.4 with six (80 registers) and 54.5 with four; 64 registers spill.
+// S = 2048: 66 KB of shared memory a block of 256 threads, three of them.
 template <int LOGS>
 constexpr int row_min_blocks() {
-    return 5;
+    return LOGS == 11 ? 3 : 5;
 }
 
 // Blocks per prime of each pass.
@@ -502,8 +499,7 @@ __host__ __device__ constexpr uint32_t col_blocks(uint32_t logS) {
 
 template <int LOGS>
 __host__ __device__ __forceinline__ uint32_t row_blocks(uint32_t logR) {
-    using RG = RowGeom<LOGS>;
-    return RG::G >= 2 ? (1u << logR) / RG::G : (1u << logR);
+    return (1u << logR) / RowGeom<LOGS>::G;
 }
 
 // Plain launches: grid (blocks per prime, K).
@@ -942,9 +938,7 @@ void launch_col_inv_t(const DevPoint& d, uint32_t* A, cudaStream_t st) {
 
 template <int LOGS, bool LAZY>
 void launch_row_t(const DevPoint& d, uint32_t* A, uint32_t* B, int mode, cudaStream_t st) {
-    using RG = RowGeom<LOGS>;
-    const uint32_t R = 1u << d.logR;
-    const dim3 grid(RG::G >= 2 ? R / RG::G : R, d.K);
+    const dim3 grid(row_blocks<LOGS>(d.logR), d.K);
     check(launch_pdl(k_ntt_row<LOGS, LAZY>, grid, dim3(row_threads<LOGS>()), row_smem_t<LOGS>(), st, d, A, B, mode),
           "row launch");
 }
@@ -1098,8 +1092,9 @@ int ntt_launches(const DevPoint& d) {
 
 uint32_t ntt_blocks_per_prime(int pass, uint32_t logR, uint32_t logS) {
     if (pass == kPassRow) {
-        const uint32_t G = 2048u >> logS;
-        return G >= 2 ? (1u << logR) / G : (1u << logR);
+        uint32_t n = 0;
+        with_log(logS, [&](auto s) { n = row_blocks<decltype(s)::value>(logR); });
+        return n;
     }
     return (1u << logS) >> (11 - logR);
 }

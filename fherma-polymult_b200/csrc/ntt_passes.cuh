@@ -121,24 +121,31 @@ __device__ __forceinline__ void col_global_store(uint32_t* const (&X)[NV], const
     }
 }
 
+// A row tile: G whole rows, 2048 elements, or 4096 for S = 2048, so that a row
+// always has its partner beside it: with one row a block each block brought in
+// both rows' twiddle tables (32 KB for 16 KB of residues), twice the table
+// traffic of the other lengths, and four blocks of 128 threads filled an SM's
+// shared memory.  Transform before -> after: N = 2^18, K = 71 218 -> 198 us,
+// N = 2^17, K = 140 199 -> 183, K = 36 51.4 -> 49.8.
 template <int LOGS>
 struct RowGeom {
+    static constexpr int kBits = LOGS == 11 ? 12 : 11;
+    static constexpr uint32_t kTile = 1u << kBits;
     static constexpr uint32_t S = 1u << LOGS;
-    static constexpr uint32_t G = 2048u >> LOGS;
-    static constexpr uint32_t kSlots = G >= 2 ? G : 2;
+    static constexpr uint32_t G = kTile >> LOGS;
+    static_assert(G >= 2, "rows and their partners");
+    static constexpr uint32_t kSlots = G;
     static constexpr uint32_t kStride = S + 4;                 // entries; pads rows across banks
-    static constexpr uint32_t kFlip = G >= 2 ? G / 2 : 1;
-    static constexpr uint32_t kPairsPerBlock = G >= 2 ? G / 2 : 1;
+    static constexpr uint32_t kFlip = G / 2;
+    static constexpr uint32_t kPairsPerBlock = G / 2;
 };
+template <int LOGS>
+using RowSwz = SwzRowT<RowGeom<LOGS>::kBits>;
 
 template <int LOGS>
 __device__ __forceinline__ uint32_t row_of_slot(uint32_t slot, uint32_t u0, uint32_t R) {
     using RG = RowGeom<LOGS>;
-    if constexpr (RG::G >= 2) {
-        return slot < RG::G / 2 ? u0 + slot : R - 1 - u0 - (slot - RG::G / 2);
-    } else {
-        return slot == 0 ? u0 : R - 1 - u0;
-    }
+    return slot < RG::G / 2 ? u0 + slot : R - 1 - u0 - (slot - RG::G / 2);
 }
 
 }  // namespace
