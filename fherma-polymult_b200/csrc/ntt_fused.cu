@@ -39,6 +39,12 @@ namespace {
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
+// The first arrival only says that this CTA runs: it has written nothing a peer
+// reads.
+__device__ __forceinline__ void cluster_arrive_started() {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+
 // The shared::cluster address, in CTA `rank` of this cluster, of what lies at
 // `addr` in this CTA's shared memory.
 __device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
@@ -114,7 +120,7 @@ __global__ void __launch_bounds__(ClusterGeom<LOGS>::T, ClusterGeom<LOGS>::kBloc
     __syncthreads();
     if (threadIdx.x < 32) row_tables_copy<LOGS>(tf, d, j, u0, bar);
     __syncwarp();
-    cluster_arrive();   // waited for before the first store to a peer: it has started
+    cluster_arrive_started();   // waited for before the first store to a peer
     const PrimeConsts pc = d.pc[j];
     const uint32_t p = pc.p;
     constexpr size_t N = size_t(1) << (LOGR + LOGS);
