@@ -49,11 +49,12 @@
 // the epilogue several times slower.
 // One epilogue loop serves every limb count (B200, us per launch, before ->
 // after, a copy unrolled per limb count before): L = 4 at N = 65536 18.4 -> 8.6,
-// L = 16 22.3 -> 9.8, L = 32 at N = 2^18 106 -> 55, L = 55 at N = 65536
+// L = 16 22.3 -> 9.8, L = 32 at N = 2^18 106 -> 42, L = 55 at N = 65536
 // 32.9 -> 20.8 (rows that start off a 16-byte boundary now leave as 16-byte
-// stores too), L = 64 26.2 -> 25.6.  What bounds it is the latency of the
-// stagers and of the epilogue's chain, not memory (53 MB in 25.6 us at L = 64)
-// or the tensor cores.
+// stores too).  What bounds it is the latency of the stagers and of the
+// epilogue's chain, not memory (53 MB in 24.2 us at L = 64) or the tensor cores
+// (20% active): four tiles a CTA take 24.8 us, 17.0 without the epilogue, 14.1
+// without the stagers' sums too; one tile 10.5, 6.7 and 5.7.
 //
 // Every wait is bounded (DevPoint::wait_ns); a timeout raises an abort flag
 // that every role checks, the copy and MMA issuers wait out what they have in
