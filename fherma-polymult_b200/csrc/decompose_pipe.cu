@@ -213,11 +213,13 @@ __device__ __forceinline__ auto fold_consts(const DecConsts& fc, int j) {
 // CTAs [0, split) take operand 0 (la -> ra), [split, gridDim.x) operand 1.
 // P: primes per fold warp and chunk.
 // RAW: rows that are not whole 16-byte groups, in a raw ring.
+// parts > 1 (few tiles): each tile is `parts` CTAs' work, part i taking the 4 P
+// primes from 4 P i of the image's (whose chunks hold fc.piece / P such runs).
 template <int P, bool LAZY, bool RAW>
 __global__ void __launch_bounds__(kThreads, 1)
     k_decompose_pipe(DevPoint d, const __grid_constant__ DecConsts fc, const uint32_t* __restrict__ la,
                      const uint32_t* __restrict__ lb, uint32_t* __restrict__ ra, uint32_t* __restrict__ rb,
-                     int operand0, uint32_t n_begin, uint32_t n_end, uint32_t split, Rings rings) {
+                     int operand0, uint32_t n_begin, uint32_t n_end, uint32_t split, uint32_t parts, Rings rings) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     pdl_launch_dependents();
     // The 128-byte swizzle is a function of the shared address: the
@@ -227,9 +229,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         return;
     }
     const uint32_t kb = d.dec_kb;
-    const int nch = static_cast<int>(fc.chunks);
+    const int nch = parts > 1 ? 1 : static_cast<int>(fc.chunks);
     constexpr uint32_t cols = 16 * P;
-        // (The shuffle tells the compiler that the warp index is uniform.)
+    // (The shuffle tells the compiler that the warp index is uniform.)
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int L = d.L, K = d.K;
     const Smem sm = carve(smem_raw, kb, nch, cols, L, rings);
@@ -239,7 +241,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t* limbs = second ? lb : la;
     uint32_t* res = second ? rb : ra;
     const uint8_t* img = fc.img[operand];
-    const uint32_t g0 = second ? split : 0, gs = second ? gridDim.x - split : split;
+    // This CTA's place among its operand's: part of every tile, first tile, step.
+    const uint32_t place = blockIdx.x - (second ? split : 0), places = second ? gridDim.x - split : split;
+    const uint32_t part = parts > 1 ? place % parts : 0, t0 = parts > 1 ? place / parts : place;
+    const uint32_t ts = parts > 1 ? places / parts : places;
     const uint32_t tiles = (n_end - n_begin + kRows - 1) / kRows;
     const uint32_t chunk_bytes = static_cast<uint32_t>(sw128_bytes(cols, kb));
     const uint64_t lim = d.wait_ns;
@@ -267,8 +272,17 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t total = static_cast<uint32_t>(b_bytes(kb, nch, cols));
         if (!(d.fault & kFaultDecompose)) {
             tc::mbar_arrive_expect_tx(sm.b_full, total);
-            for (uint32_t off = 0; off < total; off += chunk_bytes)
-                tc::bulk_g2s(sm.b + off, img + off, chunk_bytes, sm.b_full);
+            if (parts == 1) {
+                for (uint32_t off = 0; off < total; off += chunk_bytes)
+                    tc::bulk_g2s(sm.b + off, img + off, chunk_bytes, sm.b_full);
+            } else {
+                // The part's columns of the image chunk that holds them, one
+                // run per 128 K bytes.
+                const uint32_t img_cols = 16 * fc.piece, first = part * P;
+                const uint8_t* src = img + (first / fc.piece) * sw128_bytes(img_cols, kb) + (first % fc.piece) * 16 * 128;
+                for (uint32_t off = 0; off < total; off += cols * 128, src += img_cols * 128)
+                    tc::bulk_g2s(sm.b + off, src, cols * 128, sm.b_full);
+            }
         }
     }
     if (warp == 0) tc::tmem_alloc(sm.tmem_base, 512);
@@ -286,7 +300,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             uint64_t* last_bar = nullptr;   // the barrier of the latest commit
             uint32_t last_par = 0;
             uint32_t g = 0, s = 0, ph = 0;   // chunk count; operand slot and its phase
-            for (uint32_t t = blockIdx.x - g0; ok && t < tiles; t += gs) {
+            for (uint32_t t = t0; ok && t < tiles; t += ts) {
                 ok = tc::wait_or_abort(&sm.a_full[s], ph, sm.abort, lim);
                 if (!ok) break;
                 // The limbs came through the generic proxy (cp.async).
@@ -334,20 +348,20 @@ __global__ void __launch_bounds__(kThreads, 1)
         uint32_t s = 0, ph = 0, rs = 0, rph = 0, i = 0;
         // Lane 0 of the first loader warp requests the tiles, rings.raw ahead.
         const bool asks = m == 0;
-        uint32_t ask_t = blockIdx.x - g0, asked = 0;
+        uint32_t ask_t = t0, asked = 0;
         auto ask = [&](uint32_t slot) {
             const uint32_t r0 = n_begin + ask_t * kRows;
             const uint32_t bytes = min(kRows, n_end - r0) * 4 * static_cast<uint32_t>(L);
             tc::mbar_arrive_expect_tx(&sm.r_full[slot], bytes);
             tc::bulk_g2s(sm.raw + slot * raw_bytes(L), limbs + static_cast<size_t>(r0) * L, bytes, &sm.r_full[slot]);
-            ask_t += gs;
+            ask_t += ts;
             ++asked;
         };
         if (asks)
             for (uint32_t k = 0; k < rings.raw && ask_t < tiles; ++k) ask(k);
         __syncwarp();
         bool ok = true;
-        for (uint32_t t = blockIdx.x - g0; t < tiles; t += gs, ++i) {
+        for (uint32_t t = t0; t < tiles; t += ts, ++i) {
             const uint32_t nk = min(kRows, n_end - (n_begin + t * kRows));
             ok = tc::wait_or_abort(&sm.r_full[rs], rph, sm.abort, lim);
             if (ok && i >= slots) ok = tc::wait_or_abort(&sm.a_empty[s], ph ^ 1, sm.abort, lim);
@@ -397,7 +411,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t gbs = (G + 3) / 4;
         uint32_t i = 0, s = 0, ph = 0;
         bool ok = true;
-        for (uint32_t t = blockIdx.x - g0; t < tiles; t += gs, ++i) {
+        for (uint32_t t = t0; t < tiles; t += ts, ++i) {
             if (i >= slots) {
                 ok = tc::wait_or_abort(&sm.a_empty[s], ph ^ 1, sm.abort, lim);
                 ok = __all_sync(0xffffffffu, ok);
@@ -444,7 +458,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t m = qd * 32 + lane;
         const uint32_t tq = tmem + ((qd * 32) << 16) + piece * (4 * P);
         uint32_t g = 0;
-        for (uint32_t t = blockIdx.x - g0; t < tiles; t += gs) {
+        for (uint32_t t = t0; t < tiles; t += ts) {
             const uint32_t n0 = n_begin + t * kRows;
             const bool live = m < min(kRows, n_end - n0);
             const bool whole = n0 + qd * 32 + 32 <= n_end;   // every row of the warp is live
@@ -455,7 +469,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc::tc_fence_after();
-                const int j0 = c * (4 * P) + static_cast<int>(piece) * P;
+                const int j0 = (c + static_cast<int>(part)) * (4 * P) + static_cast<int>(piece) * P;
                 uint32_t r[4 * P];
                 tmem_read<4 * P>(tq + buf * kBufCols, r);
                 // The 2 P half-sums are formed before the buffer is released:
@@ -528,7 +542,7 @@ DecConsts make_dec_consts(const HostPlan& pl, const uint8_t* img_a, const uint8_
 namespace {
 
 using DecKernel = void (*)(DevPoint, const DecConsts, const uint32_t*, const uint32_t*, uint32_t*, uint32_t*, int,
-                           uint32_t, uint32_t, uint32_t, Rings);
+                           uint32_t, uint32_t, uint32_t, uint32_t, Rings);
 
 template <bool LAZY, bool RAW>
 DecKernel dec_kernel(uint32_t piece) {
@@ -570,16 +584,31 @@ void launch_decompose_pipe(const DevPoint& d, const DecConsts& dc, const uint32_
     uint32_t per = static_cast<uint32_t>(sms) / operands;
     if (per < 1) per = 1;
     if (per > tiles) per = tiles;
-    const uint32_t grid = per * operands;
-    const uint32_t split = operands == 2 ? per : grid;
-    const int nch = static_cast<int>(dc.chunks);
-    const uint32_t cols = 16 * dc.piece;
+    // Few tiles leave SMs idle and a CTA alone with all of a tile's primes: with
+    // primes enough (decompose_in_parts) each tile is cut into the most parts
+    // the SMs take, a run of whole primes each (pair alone, N = 1024: K = 59
+    // 4.2 -> 3.6 us, K = 138 5.8 -> 4.2).
+    const uint32_t cap = static_cast<uint32_t>(sms) / (static_cast<uint32_t>(operands) * tiles);
+    uint32_t piece = dc.piece, parts = 1;
+    if (decompose_in_parts(d)) {
+        for (uint32_t p = 2; p <= dc.piece; p += 2) {
+            const uint32_t n = dc.piece % p == 0 ? dc.chunks * (dc.piece / p) : 0;
+            if (n == 0 || n > cap) continue;
+            piece = p;
+            parts = n;
+            break;
+        }
+    }
+    const uint32_t grid = per * parts * operands;
+    const uint32_t split = operands == 2 ? per * parts : grid;
+    const int nch = parts > 1 ? 1 : static_cast<int>(dc.chunks);
+    const uint32_t cols = 16 * piece;
     const Rings rings = ring_sizes(d.dec_kb, nch, cols, d.L, (tiles + per - 1) / per);
     const DecKernel kernel =
-        rings.raw ? (dc.lazy_out ? dec_kernel<true, true>(dc.piece) : dec_kernel<false, true>(dc.piece))
-                  : (dc.lazy_out ? dec_kernel<true, false>(dc.piece) : dec_kernel<false, false>(dc.piece));
+        rings.raw ? (dc.lazy_out ? dec_kernel<true, true>(piece) : dec_kernel<false, true>(piece))
+                  : (dc.lazy_out ? dec_kernel<true, false>(piece) : dec_kernel<false, false>(piece));
     check(launch_pdl(kernel, dim3(grid), dim3(kThreads), smem_bytes(d.dec_kb, nch, cols, d.L, rings), st, d, dc, a, b ? b : a, A,
-                     B ? B : A, operand0, n_begin, n_end, split, rings),
+                     B ? B : A, operand0, n_begin, n_end, split, parts, rings),
           "decompose launch");
 }
 

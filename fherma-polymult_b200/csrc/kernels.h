@@ -122,6 +122,13 @@ struct DecConsts {
     uint32_t piece;             // primes per fold warp and chunk: 2, 4 .. 16
     uint32_t lazy_out;          // 1: residues below 4p (congruent), for lazy first butterflies
 };
+// Whether a product of few tiles and many primes has its tiles cut by primes
+// over the idle SMs.  Its one-block transform then finds no SM free under the
+// decompose's tail and is launched after it; with fewer primes the early launch
+// is worth more (product us, cut | not: N = 1024 K = 22 10.3 | 10.0, K = 59
+// 11.3 | 11.7, K = 138 16.0 | 17.9, N = 2048 K = 59 12.6 | 13.3, K = 138 18.2 | 21.6,
+// N = 256 K = 48 10.9 | 10.5).
+inline bool decompose_in_parts(const DevPoint& d) { return d.N >= 512 && d.N <= 2048 && d.K >= 48; }
 DecConsts make_dec_consts(const HostPlan& pl, const uint8_t* img_a, const uint8_t* img_b);
 bool decompose_pipe_supported(const HostPlan& pl);
 void decompose_pipe_init_attributes();
