@@ -391,9 +391,25 @@ void cluster_attrs() {
         check(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "cluster size");
 }
 
+// (Also loads the kernel, so that its first launch may be under capture.)
+template <int LOGN, bool LAZY>
+void whole_attrs() {
+    check(cudaFuncSetAttribute(k_ntt_whole<LOGN, LAZY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(WholeGeom<LOGN>::kSmem)),
+          "one-block smem");
+}
+
 }  // namespace
 
 void ntt_fused_init_attributes() {
+    whole_attrs<8, true>();
+    whole_attrs<9, true>();
+    whole_attrs<10, true>();
+    whole_attrs<11, true>();
+    whole_attrs<8, false>();
+    whole_attrs<9, false>();
+    whole_attrs<10, false>();
+    whole_attrs<11, false>();
     cluster_attrs<6, true>();
     cluster_attrs<7, true>();
     cluster_attrs<8, true>();
