@@ -284,10 +284,18 @@ void Engine::launch_crt_any(const DevPoint& d, const uint32_t* d_y, uint32_t* d_
     }
 }
 
+// The word is clear when this returns: run_host reads it on streams that do
+// not wait for the default stream, where a memset may be queued behind anything
+// the caller put there (and clear a later product's error).
+void Engine::clear_error() {
+    check(cudaMemsetAsync(dp_.err, 0, sizeof(uint32_t), stream_), "clear error word");
+    check(cudaStreamSynchronize(stream_), "clear error word");
+}
+
 uint32_t Engine::take_error() {
     uint32_t e = 0;
     check(cudaMemcpy(&e, dp_.err, sizeof(e), cudaMemcpyDeviceToHost), "read error word");
-    if (e) check(cudaMemset(dp_.err, 0, sizeof(e)), "clear error word");
+    if (e) clear_error();
     return e;
 }
 
@@ -518,7 +526,7 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c, uint32_
         check(cudaEventSynchronize(out_ev[nch - 1]), "copy out");
     }
     if (const uint32_t e = *herr_) {
-        check(cudaMemset(dp_.err, 0, sizeof(uint32_t)), "clear error word");
+        clear_error();
         throw PipelineTimeout("a kernel pipeline wait ran out of time (error word " + std::to_string(e) +
                               "); this product's result is not valid");
     }

@@ -110,6 +110,7 @@ private:
                     cudaStream_t st);
     void launch_crt_any(const DevPoint& d, const uint32_t* d_y, uint32_t* d_c, uint32_t n0, uint32_t n1,
                         cudaStream_t st) const;
+    void clear_error();
     void ensure_host_path();
     uint32_t* staging(uint32_t*& h);
     void set_chunks(int want);
