@@ -67,16 +67,27 @@ int enqueue_grouped(const std::vector<GroupedProduct>& prods_, const BatchSchedu
     if (sched_.order == 1) {
         std::stable_sort(ord.begin(), ord.end(), [&](size_t x, size_t y) { return prods_[x].cost > prods_[y].cost; });
     }
-    // Products by transform geometry; N <= 2048 runs the one-block-per-prime
+    // Products by transform geometry; N <= 1024 runs the one-block-per-prime
     // kernels, product by product.
     std::map<TransformClass, std::vector<size_t>> classes;
     std::vector<size_t> small;
     for (size_t i : ord) {
         const DevPoint& d = prods_[i].d;
-        if (d.logR == 0) {
+        if (d.logN <= kSmallLogN) {
             small.push_back(i);
         } else {
             classes[TransformClass{d.logR, d.logS, d.lazy != 0}].push_back(i);
+        }
+    }
+    // A single product of N = 2048 (no column passes) takes its own kernel too:
+    // 32.9 us against 34.9 for a batch of one (W = 512); two of them, one behind
+    // the other, are already slower, 36.9.
+    for (auto it = classes.begin(); it != classes.end();) {
+        if (it->first.logR == 0 && it->second.size() == 1) {
+            small.push_back(it->second[0]);
+            it = classes.erase(it);
+        } else {
+            ++it;
         }
     }
     TableFill fill;
@@ -457,7 +468,7 @@ void Batch::build_graph() {
     size_t classes = 0;
     std::vector<uint32_t> seen;
     for (const GroupedProduct& p : prods_) {
-        if (p.d.logR == 0) continue;
+        if (p.d.logN <= kSmallLogN) continue;
         const uint32_t key = p.d.logR * 64 + p.d.logS * 2 + (p.d.lazy ? 1 : 0);
         if (std::find(seen.begin(), seen.end(), key) != seen.end()) continue;
         seen.push_back(key);

@@ -67,6 +67,10 @@ void build_row_tables(const DevPoint& d, uint2* out, cudaStream_t st);
 bool ntt_fused_ok(const DevPoint& d, int mode, int sms);
 void launch_ntt_fused(const DevPoint& d, uint32_t* A, uint32_t* B, int mode, int sms, cudaStream_t st);
 void build_whole_tables(const DevPoint& d, uint2* out, cudaStream_t st);
+// The grouped form for N = 2048 (launch_ntt_group's for logR = 0), or with
+// `occupancy` its resident blocks per SM.
+struct GroupTable;
+void ntt_whole_group(const GroupTable* t, bool lazy, uint32_t grid, cudaStream_t st, int* occupancy);
 void ntt_fused_init_attributes();
 
 // The same on the tensor cores.
@@ -145,7 +149,7 @@ uint32_t ntt_blocks_per_prime(int pass, uint32_t logR, uint32_t logS);
 void launch_decompose_tc_group(const GroupTable& t, cudaStream_t st);
 void launch_crt_tc_group(const GroupTable& t, cudaStream_t st);
 // pass kPassColFwd / kPassRow (product) / kPassColInv over items of one
-// (logR, logS); grid 0 = one block per tile, else a persistent grid.
+// (logR, logS), N >= 2048 (N = 2048, logR = 0, has a row pass only); grid 0 = one block per tile, else a persistent grid.
 void launch_ntt_group(const GroupTable& t, int pass, uint32_t logR, uint32_t logS, bool lazy, uint32_t grid,
                       cudaStream_t st);
 int ntt_group_occupancy(int pass, uint32_t logR, uint32_t logS, bool lazy);

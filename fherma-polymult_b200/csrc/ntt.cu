@@ -779,6 +779,10 @@ void with_cols(uint32_t logR, uint32_t logS, F&& f) {
 template <bool LAZY>
 void group_pass(const GroupTable* t, int pass, uint32_t logR, uint32_t logS, uint32_t grid, cudaStream_t st,
                 int* occupancy) {
+    if (logR == 0 && logS == 11 && pass == kPassRow) {   // N = 2048: a block per prime
+        ntt_whole_group(t, LAZY, grid, st, occupancy);
+        return;
+    }
     auto run = [&](auto kernel, int threads, size_t smem) {
         if (occupancy) {
             check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(occupancy, kernel, threads, smem), "occupancy");
@@ -1091,6 +1095,7 @@ int ntt_launches(const DevPoint& d) {
 }
 
 uint32_t ntt_blocks_per_prime(int pass, uint32_t logR, uint32_t logS) {
+    if (logR == 0) return 1;
     if (pass == kPassRow) {
         uint32_t n = 0;
         with_log(logS, [&](auto s) { n = row_blocks<decltype(s)::value>(logR); });

@@ -22,6 +22,7 @@
 // Twiddle tables come in by bulk copies under the preceding kernel's tail.  The
 // arithmetic is that of the separate passes (ntt.cu), so the residues y_j are
 // the same words.
+#include "group.cuh"
 #include "kernels.h"
 #include "ntt_passes.cuh"
 #include "pdl.cuh"
@@ -332,6 +333,89 @@ __global__ void __launch_bounds__(2 * WholeGeom<LOGN>::T) k_ntt_whole(DevPoint d
     }
 }
 
+// The products of N = 2048 of a batch in one launch: a (possibly persistent)
+// grid walks the table's blocks, one a prime.  A batch has blocks enough for
+// throughput to count, so one group of N / 16 threads holds both operands (a
+// twiddle load serves both, and no thread idles through the inverse rounds).
+// Batch of 32, us: one launch a product, each behind the one before, 171 at
+// W = 128 and 278 at W = 2048; one launch, two groups a block 65.7 and 209;
+// this 65.0 and 187.
+template <bool LAZY>
+__global__ void __launch_bounds__(WholeGeom<11>::T, 5) k_ntt_whole_group(const __grid_constant__ GroupTable t) {
+    extern __shared__ __align__(1024) uint32_t smem[];
+    constexpr int LOGN = 11;
+    using WG = WholeGeom<LOGN>;
+    constexpr int RB = WG::RB, E = WG::E;
+    constexpr uint32_t N = WG::N;
+    using SWZ = SwzRowT<LOGN>;
+    using RPW = RP<LOGN, 0, SWZ, RB>;
+    constexpr int last = RPW::kCount - 1, sh = RPW::lo(0);
+    uint32_t* const tiles[2] = {smem, smem + N};
+    uint2* tf = reinterpret_cast<uint2*>(smem + 2 * N);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(tf + N);
+    const RowTable<LOGN, 0, false, 0> fw{tf};
+    const RowTable<LOGN, 0, true, 0> iw{tf};
+    if (threadIdx.x == 0) {
+        tc::mbar_init(bar, 1);
+        tc::fence_mbar_init();
+    }
+    __syncthreads();
+    uint32_t phase = 0;
+    for (uint32_t b = blockIdx.x; b < t.total; b += gridDim.x, phase ^= 1) {
+        if (b != blockIdx.x) __syncthreads();   // the previous prime's tiles and table
+        const uint32_t i = group_locate(t, b);
+        const GroupItem& it = t.item[i];
+        const size_t j = it.j0 + (b - t.first[i]);
+        if (threadIdx.x == 0) {
+            tc::mbar_arrive_expect_tx(bar, N * sizeof(uint2));
+            tc::bulk_g2s(tf, it.d.row_tw + j * N, N * sizeof(uint2), bar);
+        }
+        const PrimeConsts pc = it.d.pc[j];
+        const uint32_t p = pc.p;
+        uint32_t* const X[2] = {it.A + j * N, it.B + j * N};
+        {
+            const uint32_t base = round_base<LOGN, 0, SWZ, RB, 0>(threadIdx.x);
+            uint32_t v[2][E];
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+#pragma unroll
+                for (int k = 0; k < E; ++k) v[o][k] = X[o][base | (k << sh)];
+            }
+            if (!tc::wait_parity(bar, phase, it.d.wait_ns) && (threadIdx.x & 31) == 0) atomicOr(it.d.err, 4u);
+            fwd_round<LOGN, 0, SWZ, RB, 0, LAZY, 2>(v, base, fw, p);
+#pragma unroll
+            for (int o = 0; o < 2; ++o) store_round<LOGN, 0, SWZ, RB, 0>(tiles[o], v[o], base);
+            __syncthreads();
+        }
+        fwd_range<LOGN, 0, SWZ, RB, 1, last, LAZY, 2>(tiles, fw, p);
+        {
+            const uint32_t base = round_base<LOGN, 0, SWZ, RB, last>(threadIdx.x);
+            uint32_t v[2][E];
+#pragma unroll
+            for (int o = 0; o < 2; ++o) load_round<LOGN, 0, SWZ, RB, last>(tiles[o], v[o], base);
+            fwd_round<LOGN, 0, SWZ, RB, last, LAZY, 2>(v, base, fw, p);
+#pragma unroll
+            for (int k = 0; k < E; ++k) v[0][k] = pointwise<LAZY>(v[0][k], v[1][k], pc);
+            inv_round<LOGN, 0, SWZ, RB, last, LAZY, true>(v[0], base, iw, p);
+            store_round<LOGN, 0, SWZ, RB, last>(tiles[0], v[0], base);
+            __syncthreads();
+        }
+        inv_range<LOGN, 0, SWZ, RB, last - 1, 1, LAZY, true>(tiles[0], iw, p);
+        {
+            const uint32_t base = round_base<LOGN, 0, SWZ, RB, 0>(threadIdx.x);
+            uint32_t v[E];
+            load_round<LOGN, 0, SWZ, RB, 0>(tiles[0], v, base);
+            inv_round<LOGN, 0, SWZ, RB, 0, LAZY, true>(v, base, iw, p);
+            if constexpr (LAZY) {
+#pragma unroll
+                for (int k = 0; k < E; ++k) v[k] = reduce_once(v[k], p);
+            }
+#pragma unroll
+            for (int k = 0; k < E; ++k) X[0][base | (k << sh)] = v[k];
+        }
+    }
+}
+
 // Round-major tables of the one-CTA transforms from the plan's entry-order ones.
 __global__ void __launch_bounds__(256) k_whole_tables(DevPoint d, int rb, uint2* out) {
     const size_t at = static_cast<size_t>(blockIdx.x) * d.N;
@@ -399,9 +483,33 @@ void whole_attrs() {
           "one-block smem");
 }
 
+template <bool LAZY>
+void whole_group_attrs() {
+    check(cudaFuncSetAttribute(k_ntt_whole_group<LAZY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(WholeGeom<11>::kSmem)),
+          "one-block smem");
+}
+
+template <bool LAZY>
+void whole_group(const GroupTable* t, uint32_t grid, cudaStream_t st, int* occupancy) {
+    using WG = WholeGeom<11>;
+    if (occupancy) {
+        check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(occupancy, k_ntt_whole_group<LAZY>, WG::T, WG::kSmem),
+              "occupancy");
+    } else {
+        k_ntt_whole_group<LAZY><<<grid, WG::T, WG::kSmem, st>>>(*t);
+    }
+}
+
 }  // namespace
 
+void ntt_whole_group(const GroupTable* t, bool lazy, uint32_t grid, cudaStream_t st, int* occupancy) {
+    lazy ? whole_group<true>(t, grid, st, occupancy) : whole_group<false>(t, grid, st, occupancy);
+}
+
 void ntt_fused_init_attributes() {
+    whole_group_attrs<true>();
+    whole_group_attrs<false>();
     whole_attrs<8, true>();
     whole_attrs<9, true>();
     whole_attrs<10, true>();
