@@ -643,7 +643,13 @@ __global__ void __launch_bounds__(256, 3) k_ntt_row_mixed(const __grid_constant_
     uint32_t uses[2] = {0, 0};   // every thread counts both regions' uses
     const uint32_t half = threadIdx.x >> 7;
     for (uint32_t b = blockIdx.x; b < t.total; b += gridDim.x) {
-        if (b != blockIdx.x) __syncthreads();
+        if (b != blockIdx.x) {
+            // Tiles of different row lengths lie differently: the bulk copies of
+            // this one's tables may go where the one before kept residues, which
+            // were written by plain stores.
+            tc::fence_proxy_async_smem();
+            __syncthreads();
+        }
         const uint32_t i = group_locate(t, b);
         const GroupItem& it = t.item[i];
         const uint32_t local = b - t.first[i];
