@@ -362,17 +362,6 @@ __device__ __forceinline__ size_t row_offset(uint32_t i, uint32_t u0, uint32_t R
     return static_cast<size_t>(row_of_slot<LOGS>(i >> LOGS, u0, R)) * (1u << LOGS) + (i & ((1u << LOGS) - 1u));
 }
 
-template <int LOGS>
-constexpr int row_threads() {
-    return 1 << (RowGeom<LOGS>::kBits - row_pass_rb(LOGS));
-}
-
-// The row pass's tables barrier sits after the tiles and the tables.
-template <int LOGS>
-constexpr size_t row_bar_offset() {
-    return 2 * RowGeom<LOGS>::kTile * sizeof(uint32_t) + RowGeom<LOGS>::kSlots * RowGeom<LOGS>::kStride * sizeof(uint2);
-}
-
 // phase: parity of this tile's use of the tables barrier (the block's tile
 // count so far, mod 2); the barrier is initialised by the kernel.
 // smem: this team's region (row_smem_t<LOGS>() bytes, 1024-byte aligned);
@@ -583,9 +572,10 @@ __global__ void __launch_bounds__(row_threads<LOGS>(), (row_min_blocks<LOGS>()))
 // Grouped passes over products of mixed row lengths (every item R = 64:
 // N = 2^12 .. 2^17, one prime window): one launch per pass for a whole batch.
 // The column passes switch on the item's row length; the row pass runs
-// 256-thread blocks, one tile per block for 8-element rounds and two
-// 128-thread tiles per block (HalfTeam, named barriers, a shared-memory region
-// and tables barrier each) for 16-element rounds.
+// 256-thread blocks, one tile per block where its threads are 256 (8-element
+// rounds, and the 4096-element tiles of S = 2048) and two 128-thread tiles per
+// block (HalfTeam, named barriers, half of the shared memory and a tables
+// barrier each) for the other 16-element rounds.
 
 template <class F>
 __device__ __forceinline__ void with_row_log(uint32_t logS, F&& f) {
@@ -625,15 +615,16 @@ __global__ void __launch_bounds__(256, 6) k_ntt_col_inv_mixed(const __grid_const
     }
 }
 
-// Shared memory: two regions of `region` bytes, each ending in its tables
-// barrier.  Block b of item i: tile local(b) (one per block) or tiles
-// 2 local(b) + half (two per block), tile = (prime, row block).
+// Shared memory: the tables barriers' 32 bytes, aligned, past `bytes` of tiles
+// and tables, which a 256-thread tile has to itself and two 128-thread tiles
+// halve (mixed_row_bytes).  Block b of item i: tile local(b) (one per block) or
+// tiles 2 local(b) + half (two per block), tile = (prime, row block).
 template <bool LAZY>
-__global__ void __launch_bounds__(256, 3) k_ntt_row_mixed(const __grid_constant__ GroupTable t, uint32_t region) {
+__global__ void __launch_bounds__(256, 3) k_ntt_row_mixed(const __grid_constant__ GroupTable t, uint32_t bytes) {
     extern __shared__ __align__(1024) uint32_t smem[];
     uint8_t* base = reinterpret_cast<uint8_t*>(smem);
-    uint64_t* tbar[2] = {reinterpret_cast<uint64_t*>(base + region - 16),
-                         reinterpret_cast<uint64_t*>(base + 2 * region - 16)};
+    uint64_t* bars = reinterpret_cast<uint64_t*>(base + bytes);
+    uint64_t* tbar[2] = {bars, bars + 2};
     if (threadIdx.x == 0) {
         tc::mbar_init(tbar[0], 1);
         tc::mbar_init(tbar[1], 1);
@@ -663,7 +654,7 @@ __global__ void __launch_bounds__(256, 3) k_ntt_row_mixed(const __grid_constant_
             } else {
                 const uint32_t tile = 2 * local + half;
                 row_body<LS, LAZY, HalfTeam>(it.d, it.A, it.B, kRowProduct, it.j0 + tile / per, tile % per,
-                                             uses[half] & 1, reinterpret_cast<uint32_t*>(base + half * region),
+                                             uses[half] & 1, reinterpret_cast<uint32_t*>(base + half * (bytes / 2)),
                                              tbar[half]);
                 ++uses[0];
                 ++uses[1];
@@ -989,14 +980,6 @@ uint32_t ntt_mixed_blocks(int pass, uint32_t logS, uint32_t primes) {
 
 namespace {
 
-uint32_t row_mixed_region(uint32_t max_log_s) {
-    size_t r = 0;
-    for (uint32_t ls = 6; ls <= max_log_s && ls <= 11; ++ls) {
-        with_log(ls, [&](auto l) { r = std::max(r, row_smem_t<decltype(l)::value>()); });
-    }
-    return static_cast<uint32_t>((r + 1023) / 1024 * 1024);
-}
-
 template <bool LAZY>
 void mixed_pass(const GroupTable* t, int pass, uint32_t max_log_s, uint32_t grid, cudaStream_t st, int* occupancy) {
     auto run = [&](auto kernel, size_t smem, auto... extra) {
@@ -1011,8 +994,8 @@ void mixed_pass(const GroupTable* t, int pass, uint32_t max_log_s, uint32_t grid
     } else if (pass == kPassColInv) {
         run(k_ntt_col_inv_mixed<LAZY>, col_inv_smem_t(6));
     } else if (pass == kPassRow) {
-        const uint32_t region = row_mixed_region(max_log_s);
-        run(k_ntt_row_mixed<LAZY>, 2 * size_t(region), region);
+        const uint32_t bytes = mixed_row_bytes(max_log_s);
+        run(k_ntt_row_mixed<LAZY>, bytes + 32, bytes);
     } else {
         throw std::runtime_error("mixed transform: unknown pass");
     }
@@ -1027,7 +1010,7 @@ void mixed_attrs() {
                                static_cast<int>(col_inv_smem_t(6))),
           "mixed smem");
     check(cudaFuncSetAttribute(k_ntt_row_mixed<LAZY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(2 * row_mixed_region(11))),
+                               static_cast<int>(mixed_row_bytes(11) + 32)),
           "mixed smem");
 }
 

@@ -148,6 +148,35 @@ __device__ __forceinline__ uint32_t row_of_slot(uint32_t slot, uint32_t u0, uint
     return slot < RG::G / 2 ? u0 + slot : R - 1 - u0 - (slot - RG::G / 2);
 }
 
+template <int LOGS>
+constexpr int row_threads() {
+    return 1 << (RowGeom<LOGS>::kBits - row_pass_rb(LOGS));
+}
+
+// The row pass's tables barrier sits after the tiles and the tables.
+template <int LOGS>
+constexpr size_t row_bar_offset() {
+    return 2 * RowGeom<LOGS>::kTile * sizeof(uint32_t) + RowGeom<LOGS>::kSlots * RowGeom<LOGS>::kStride * sizeof(uint2);
+}
+
+// Bytes of tiles and tables of a mixed-geometry row block for rows up to
+// 2^max_log_s: room for one 256-thread tile or, in halves, two 128-thread ones.
+// (With a region the size of the largest tile for each half, S = 2048 took 130
+// KB, one block an SM: N = 2^17, 2^16, 2^14 and 2^13 in one batch 295 us, with
+// this 262; before there were such tiles 266.)
+constexpr uint32_t mixed_row_bytes(uint32_t max_log_s) {
+    const int threads[6] = {row_threads<6>(), row_threads<7>(), row_threads<8>(),
+                            row_threads<9>(), row_threads<10>(), row_threads<11>()};
+    const size_t need[6] = {row_bar_offset<6>(), row_bar_offset<7>(), row_bar_offset<8>(),
+                            row_bar_offset<9>(), row_bar_offset<10>(), row_bar_offset<11>()};
+    size_t r = 0;
+    for (uint32_t s = 6; s <= max_log_s && s <= 11; ++s) {
+        const size_t n = threads[s - 6] == 256 ? need[s - 6] : 2 * need[s - 6];
+        r = n > r ? n : r;
+    }
+    return static_cast<uint32_t>((r + 2047) / 2048 * 2048);   // halves on 1024 bytes
+}
+
 }  // namespace
 
 }  // namespace fpm
