@@ -336,8 +336,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (!(d.fault & kFaultDecompose)) tc::wait_parity(sm.b_full, 0, lim);
         }
         __syncwarp();
-    } else if (RAW && warp < kEpiWarp0 && (reinterpret_cast<uintptr_t>(limbs) & 15u) == 0 &&
-               (((n_end - n_begin) * static_cast<uint32_t>(L)) & 3u) == 0) {
+    } else if (RAW && warp < kEpiWarp0 &&
+               raw_tiles_aligned(reinterpret_cast<uintptr_t>(limbs), n_begin, n_end, L)) {
         // ---- loaders, rows that are not whole 16-byte groups: a tile arrives
         // as it lies in memory, one bulk copy (its rows are contiguous and, 128
         // rows a tile, start and end on 16 bytes); a thread then moves one row

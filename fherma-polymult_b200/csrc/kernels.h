@@ -133,6 +133,13 @@ struct DecConsts {
 // 11.3 | 11.7, K = 138 16.0 | 17.9, N = 2048 K = 59 12.6 | 13.3, K = 138 18.2 | 21.6,
 // N = 256 K = 48 10.9 | 10.5).
 inline bool decompose_in_parts(const DevPoint& d) { return d.N >= 512 && d.N <= 2048 && d.K >= 48; }
+// Whether [n_begin, n_end) of an N x L limb array at byte address `limbs` may come
+// in as whole 128-row tiles by bulk copies: every tile must start and end on 16
+// bytes (128 rows are whole 16-byte groups whatever L is).
+__host__ __device__ inline bool raw_tiles_aligned(uint64_t limbs, uint32_t n_begin, uint32_t n_end, int L) {
+    const uint32_t l = static_cast<uint32_t>(L);
+    return (limbs & 15u) == 0 && ((n_begin * l) & 3u) == 0 && ((n_end * l) & 3u) == 0;
+}
 DecConsts make_dec_consts(const HostPlan& pl, const uint8_t* img_a, const uint8_t* img_b);
 bool decompose_pipe_supported(const HostPlan& pl);
 void decompose_pipe_init_attributes();
