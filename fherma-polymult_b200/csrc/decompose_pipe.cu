@@ -584,20 +584,10 @@ void launch_decompose_pipe(const DevPoint& d, const DecConsts& dc, const uint32_
     uint32_t per = static_cast<uint32_t>(sms) / operands;
     if (per < 1) per = 1;
     if (per > tiles) per = tiles;
-    // Few tiles leave SMs idle and a CTA alone with all of a tile's primes: with
-    // primes enough (decompose_in_parts) each tile is cut into the most parts
-    // the SMs take, a run of whole primes each (pair alone, N = 1024: K = 59
-    // 4.2 -> 3.6 us, K = 138 5.8 -> 4.2).
-    const uint32_t cap = static_cast<uint32_t>(sms) / (static_cast<uint32_t>(operands) * tiles);
     uint32_t piece = dc.piece, parts = 1;
-    if (decompose_in_parts(d)) {
-        for (uint32_t p = 2; p <= dc.piece; p += 2) {
-            const uint32_t n = dc.piece % p == 0 ? dc.chunks * (dc.piece / p) : 0;
-            if (n == 0 || n > cap) continue;
-            piece = p;
-            parts = n;
-            break;
-        }
+    if (const DecParts cut = decompose_parts(d.N, d.K, tiles, static_cast<uint32_t>(operands), sms); cut.parts > 1) {
+        piece = cut.piece;
+        parts = cut.parts;
     }
     const uint32_t grid = per * parts * operands;
     const uint32_t split = operands == 2 ? per * parts : grid;

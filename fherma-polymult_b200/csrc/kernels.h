@@ -126,13 +126,29 @@ struct DecConsts {
     uint32_t piece;             // primes per fold warp and chunk: 2, 4 .. 16
     uint32_t lazy_out;          // 1: residues below 4p (congruent), for lazy first butterflies
 };
-// Whether a product of few tiles and many primes has its tiles cut by primes
-// over the idle SMs.  Its one-block transform then finds no SM free under the
+// Few tiles leave SMs idle and a CTA alone with all of a tile's primes: with
+// primes enough each tile is cut into the most parts the SMs take, a run of 4
+// piece primes each (pair alone, N = 1024: K = 59 4.2 -> 3.6 us, K = 138 5.8 ->
+// 4.2).  A product's one-block transform then finds no SM free under the
 // decompose's tail and is launched after it; with fewer primes the early launch
 // is worth more (product us, cut | not: N = 1024 K = 22 10.3 | 10.0, K = 59
 // 11.3 | 11.7, K = 138 16.0 | 17.9, N = 2048 K = 59 12.6 | 13.3, K = 138 18.2 | 21.6,
-// N = 256 K = 48 10.9 | 10.5).
-inline bool decompose_in_parts(const DevPoint& d) { return d.N >= 512 && d.N <= 2048 && d.K >= 48; }
+// N = 256 K = 48 10.9 | 10.5).  Not every K divides into parts that the SMs take
+// (N = 2048, K = 49 .. 56: 7 parts of 32 tiles, or one): such tiles stay whole.
+struct DecParts {
+    uint32_t parts, piece;
+};
+inline DecParts decompose_parts(uint32_t N, int K, uint32_t tiles, uint32_t operands, int sms) {
+    const uint32_t whole = dec_wide_piece(K), chunks = dec_wide_chunks(K);
+    if (N >= 512 && N <= 2048 && K >= 48) {
+        const uint32_t cap = static_cast<uint32_t>(sms) / (operands * tiles);
+        for (uint32_t p = 2; p <= whole; p += 2) {
+            const uint32_t n = whole % p == 0 ? chunks * (whole / p) : 0;
+            if (n > 0 && n <= cap) return {n, p};
+        }
+    }
+    return {1, whole};
+}
 // Whether [n_begin, n_end) of an N x L limb array at byte address `limbs` may come
 // in as whole 128-row tiles by bulk copies: every tile must start and end on 16
 // bytes (128 rows are whole 16-byte groups whatever L is).

@@ -449,11 +449,13 @@ void launch_cluster(const DevPoint& d, uint32_t* A, uint32_t* B, int sms, cudaSt
 }
 
 template <bool LAZY>
-void launch_whole(const DevPoint& d, uint32_t* A, uint32_t* B, int mode, cudaStream_t st) {
+void launch_whole(const DevPoint& d, uint32_t* A, uint32_t* B, int mode, int sms, cudaStream_t st) {
+    // Early unless the product's decompose fills the SMs (decompose_parts).
+    const bool early = decompose_parts(d.N, d.K, (d.N + 127) / 128, 2, sms).parts == 1;
     auto run = [&](auto ln) {
         using WG = WholeGeom<decltype(ln)::value>;
         check(launch_cluster_grid(k_ntt_whole<decltype(ln)::value, LAZY>, dim3(d.K), dim3(2 * WG::T), 1,
-                                  !decompose_in_parts(d), WG::kSmem, st, d, A, B, mode),
+                                  early, WG::kSmem, st, d, A, B, mode),
               "transform launch");
     };
     switch (d.logN) {
@@ -551,7 +553,7 @@ bool ntt_fused_ok(const DevPoint& d, int mode, int sms) {
 
 void launch_ntt_fused(const DevPoint& d, uint32_t* A, uint32_t* B, int mode, int sms, cudaStream_t st) {
     if (d.logN <= 11) {
-        d.lazy ? launch_whole<true>(d, A, B, mode, st) : launch_whole<false>(d, A, B, mode, st);
+        d.lazy ? launch_whole<true>(d, A, B, mode, sms, st) : launch_whole<false>(d, A, B, mode, sms, st);
     } else {
         d.lazy ? launch_cluster<true>(d, A, B, sms, st) : launch_cluster<false>(d, A, B, sms, st);
     }

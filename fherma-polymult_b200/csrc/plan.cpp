@@ -274,13 +274,9 @@ HostPlan make_plan_basis(uint32_t N, uint32_t W, int L, int qbits, int pmax_log2
     pl.dec_img_a.assign(dchunk * pl.dec_chunks, 0);
     pl.dec_img_b.assign(dchunk * pl.dec_chunks, 0);
     pl.dec_fold.resize(K);
-    // Wide images: the fewest chunks of at most 64 primes (256 GEMM columns,
-    // the MMA's widest N), all of one size: the pipeline's four fold warps per
-    // lane quadrant take a quarter of a chunk each, and a chunk costs them the
-    // same however few of its columns are used.  A quarter is an even number
-    // of primes (TMEM is read two primes at a time).
-    pl.dec_wchunks = static_cast<uint32_t>((K + 63) / 64);
-    pl.dec_wpiece = (static_cast<uint32_t>(K) + 8 * pl.dec_wchunks - 1) / (8 * pl.dec_wchunks) * 2;
+    // Wide images (dec_wide_chunks).
+    pl.dec_wchunks = dec_wide_chunks(K);
+    pl.dec_wpiece = dec_wide_piece(K);
     const uint32_t wprimes = 4 * pl.dec_wpiece, wcols = 4 * wprimes;
     const size_t wchunk = sw128_bytes(wcols, pl.dec_kb);   // 128-byte-swizzle layout (sw128_offset)
     pl.dec_wimg_a.assign(wchunk * pl.dec_wchunks, 0);

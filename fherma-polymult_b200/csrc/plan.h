@@ -35,6 +35,17 @@ constexpr uint32_t kWholeMinLogN = 8;
 constexpr uint32_t kTileLog = 11;            // 2048-element tiles
 constexpr uint32_t kTile = 1u << kTileLog;
 
+// The pipelined decompose's chunks of K primes: the fewest of at most 64 primes
+// (256 GEMM columns, the MMA's widest N), all of one size: the pipeline's four fold warps per
+// lane quadrant take a quarter of a chunk each, and a chunk costs them the
+// same however few of its columns are used.  A quarter (the piece) is an even
+// number of primes (TMEM is read two primes at a time).
+inline uint32_t dec_wide_chunks(int K) { return static_cast<uint32_t>((K + 63) / 64); }
+inline uint32_t dec_wide_piece(int K) {
+    const uint32_t c = dec_wide_chunks(K);
+    return (static_cast<uint32_t>(K) + 8 * c - 1) / (8 * c) * 2;
+}
+
 struct Geometry {
     uint32_t logN = 0, logR = 0, logS = 0;
     bool small = false;
