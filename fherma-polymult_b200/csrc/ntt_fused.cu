@@ -302,9 +302,11 @@ __global__ void __launch_bounds__(2 * WholeGeom<LOGN>::T) k_ntt_whole(DevPoint d
 #pragma unroll
             for (int k = 0; k < E; ++k) v[0][k] = canon4(v[0][k], p);
         }
-        static_assert(RPW::lo(last) == 0, "the last round's elements are adjacent");
+        // Through shared memory, so that a warp's stores are whole lines.
+        store_round<LOGN, 0, SWZ, RB, last>(tile[0], v[0], base);
+        TEAM::sync();
 #pragma unroll
-        for (int k = 0; k < E; ++k) X[base | k] = v[0][k];
+        for (int k = 0; k < E; ++k) X[tid + k * WG::T] = tile[0][SWZ::f(tid + k * WG::T)];
         return;
     }
     // B's values to A's threads, which go on alone.
