@@ -370,8 +370,9 @@ void Engine::ensure_host_path() {
     if (la_) return;
     const size_t n = words(), bytes = n * sizeof(uint32_t);
     if (!herr_) check(cudaHostAlloc(reinterpret_cast<void**>(&herr_), sizeof(uint32_t), cudaHostAllocDefault), "pinned");
-    lc_ = dalloc<uint32_t>(n);
-    lb_ = dalloc<uint32_t>(n);
+    // (A call that ran out of memory here may be tried again.)
+    if (!lc_) lc_ = dalloc<uint32_t>(n);
+    if (!lb_) lb_ = dalloc<uint32_t>(n);
     // I/O chunks: equal slices on 128-coefficient boundaries, so a chunk's
     // decompose and CRT blocks never straddle two.  Each chunk costs about
     // 13 us of launches and pipeline start-up, so the default aims at 16 MiB of
