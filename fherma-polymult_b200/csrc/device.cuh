@@ -22,7 +22,7 @@ struct DevPoint {
     const uint2* row_q_f;      // K x S
     const uint2* row_tw;       // K x R x S: row u's forward table, round-major (built once)
     const uint2* full_f;       // K x N (small transforms)
-    const uint2* full_i;
+    const uint2* full_i;       // N < 256 only
     const uint32_t* q;         // L
     double q_top;
     double q_top_inv;          // 1 / q_top, for the quotient estimate

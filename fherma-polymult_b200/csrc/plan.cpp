@@ -188,7 +188,7 @@ HostPlan make_plan_basis(uint32_t N, uint32_t W, int L, int qbits, int pmax_log2
     pl.p_recip.resize(K);
     if (g.small) {
         pl.full_f.resize(static_cast<size_t>(K) * N);
-        pl.full_i.resize(static_cast<size_t>(K) * N);
+        if (logN < kWholeMinLogN) pl.full_i.resize(static_cast<size_t>(K) * N);
     } else {
         pl.row_u_f.resize(static_cast<size_t>(K) * R * g.logS);
         pl.row_q_f.resize(static_cast<size_t>(K) * S);
@@ -238,7 +238,7 @@ HostPlan make_plan_basis(uint32_t N, uint32_t W, int L, int qbits, int pmax_log2
             for (uint32_t y = 0; y < N; ++y) {
                 const uint32_t e = bitrev(y, logN);
                 pl.full_f[static_cast<size_t>(j) * N + y] = pair(pow_mod(psi, e, p), p);
-                pl.full_i[static_cast<size_t>(j) * N + y] = pair(pow_mod(ipsi, e, p), p);
+                if (!pl.full_i.empty()) pl.full_i[static_cast<size_t>(j) * N + y] = pair(pow_mod(ipsi, e, p), p);
             }
             continue;
         }

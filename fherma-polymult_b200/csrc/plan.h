@@ -83,7 +83,9 @@ struct HostPlan {
     //   row_u_f: K x R x logS pairs, row_q_f: K x S pairs (entry 0 unused), each
     //   prime's S entries in the round-major order of row_table_pos.
     std::vector<uint2> row_u_f, row_q_f;
-    // Small transforms (logN <= kSmallLogN): psi^bitrev_logN(y), K x N pairs.
+    // Small transforms (logN <= kSmallLogN): psi^bitrev_logN(y), K x N pairs, and
+    // below 2^kWholeMinLogN the same of psi^-1 (k_ntt_whole reads forward tables
+    // only).
     std::vector<uint2> full_f, full_i;
 
     // CRT: M_j = P / p_j mod q (K x L), negvP_v = -v P mod q ((K + 1) x L),
