@@ -71,6 +71,7 @@ void build_whole_tables(const DevPoint& d, uint2* out, cudaStream_t st);
 // `occupancy` its resident blocks per SM.
 struct GroupTable;
 void ntt_whole_group(const GroupTable* t, bool lazy, uint32_t grid, cudaStream_t st, int* occupancy);
+void ntt_whole_group_init_attributes();
 void ntt_fused_init_attributes();
 
 // The same on the tensor cores.

@@ -511,9 +511,12 @@ void ntt_whole_group(const GroupTable* t, bool lazy, uint32_t grid, cudaStream_t
     lazy ? whole_group<true>(t, grid, st, occupancy) : whole_group<false>(t, grid, st, occupancy);
 }
 
-void ntt_fused_init_attributes() {
+void ntt_whole_group_init_attributes() {
     whole_group_attrs<true>();
     whole_group_attrs<false>();
+}
+
+void ntt_fused_init_attributes() {
     whole_attrs<8, true>();
     whole_attrs<9, true>();
     whole_attrs<10, true>();
