@@ -40,21 +40,25 @@
 //     thread per row: a quotient estimate e from the top TMEM columns (within
 //     one of floor(X / q)), then one pass from the bottom limb up that
 //     assembles X from D with carries, subtracts e q, stores the limbs of its
-//     row and tracks the borrows that tell whether X - e q lies in [0, q); the
-//     rare row that does not (about 2^-11 of them) adds or subtracts q in a
-//     second pass over what it stored.
+//     row and tracks the borrows that tell whether X - e q lies in [0, q).  A
+//     row whose estimate lies within 2^-8 of an integer (2^-7 of uniform rows) or
+//     that came out negative takes a second pass over what it stored, which
+//     compares and adds or subtracts q.  Results that are small numbers or q
+//     minus small numbers send every row there: with operands all q - 1 this
+//     kernel takes 37.3 us for 19.8 at N = 65536, W = 1747, 51.3 for 22.8 at
+//     W = 2048.
 // Per-prime constants and q come in as kernel parameters and are copied to
 // shared memory at the start: read from the parameter bank inside the loops
 // (a few KB swept by every chunk and every limb) they made the stagers and
 // the epilogue several times slower.
-// One epilogue loop serves every limb count (B200, us per launch, before ->
-// after, a copy unrolled per limb count before): L = 4 at N = 65536 18.4 -> 8.6,
-// L = 16 22.3 -> 9.8, L = 32 at N = 2^18 106 -> 42, L = 55 at N = 65536
-// 32.9 -> 20.8 (rows that start off a 16-byte boundary now leave as 16-byte
-// stores too).  What bounds it is the latency of the stagers and of the
-// epilogue's chain, not memory (53 MB in 24.2 us at L = 64) or the tensor cores
-// (20% active): four tiles a CTA take 24.8 us, 17.0 without the epilogue, 14.1
-// without the stagers' sums too; one tile 10.5, 6.7 and 5.7.
+// One epilogue loop serves every limb count: L = 4 at N = 65536 8.6 us a launch,
+// L = 16 9.8, L = 55 20.8, where a copy of it unrolled over the limbs took 18.4,
+// 22.3 and 32.9 (and stored rows that start off a 16-byte boundary word by word).
+// What bounds it is the latency of the stagers and of the epilogue's chain, not
+// memory (53 MB in 23.6 us at L = 64) or the tensor cores (20% active): four
+// tiles a CTA took 24.8 us, 17.0 without the epilogue, 14.1 without the stagers'
+// sums too; one tile 10.5, 6.7 and 5.7 (before the rounding sum lost its shifts,
+// 1 us at L = 64).
 //
 // Every wait is bounded (DevPoint::wait_ns); a timeout raises an abort flag
 // that every role checks, the copy and MMA issuers wait out what they have in

@@ -27,16 +27,15 @@
 //     p_j and store the residues (a warp writes 32 consecutive words per
 //     prime).
 // What bounds it at L = 64 is the fold warps' way through a chunk: TMEM reads,
-// folds, stores (106 MB in 23.8 us at K = 139; 16 us without them).  So every fold warp gets the same
-// share of every chunk (K = 139 is 3 chunks of 48 with 12 primes a warp; as 64 +
-// 64 + 11, 16 a warp, the last chunk took as long as a full one), warps whose
-// rows and primes all exist store without a test per prime, and a store's
-// address is one 32-bit add.  Pair launch, before -> after: K = 139 at
-// N = 65536 33.4 -> 25.3 us, K = 71 at N = 2^18 68.0 -> 47.6, K = 36 at
-// N = 2^17 21.7 -> 17.3, K = 60 at N = 32768 9.0 -> 8.2.  The fold constants
-// stay in the parameter bank: from shared memory, which the MMAs load heavily,
-// they took K = 60 from 8.2 to 9.1 us (and K = 139 from 25.3 to 24.4).  (Figures
-// of that step; the ring's and the fold's are beside them below.)
+// folds, stores (106 MB in 23.8 us at K = 139; 16 us without them).  So every
+// fold warp gets the same share of every chunk (K = 139 is 3 chunks of 48 with 12
+// primes a warp; as 64 + 64 + 11, 16 a warp, the last chunk took as long as a
+// full one), warps whose rows and primes all exist store without a test per
+// prime, and a store's address is one 32-bit add: together 25.3 us where unequal
+// chunks took 33.4 (K = 71 at N = 2^18 47.6 for 68.0, K = 60 at N = 32768 8.2 for
+// 9.0, all before the rings and the fold below).  The fold constants stay in the
+// parameter bank: from shared memory, which the MMAs load heavily, they took
+// K = 60 from 8.2 to 9.1 us (and K = 139 from 25.3 to 24.4).
 // The fold constants come from kernel parameters.  Every wait is bounded
 // (DevPoint::wait_ns); a timeout raises an abort flag that every role checks,
 // and the error word gets bit 0.
@@ -525,8 +524,9 @@ DecConsts make_dec_consts(const HostPlan& pl, const uint8_t* img_a, const uint8_
     dc.img[1] = img_b;
     dc.chunks = pl.dec_wchunks;
     dc.piece = pl.dec_wpiece;
-    // The four-step transforms start with lazy butterflies; the one-block
-    // transform (N <= 1024) and the full-reduction window want canonical input.
+    // Transforms of N >= 2048 start with lazy butterflies; k_ntt_small (N < 256)
+    // and the full-reduction window want canonical input, and N = 256 .. 1024,
+    // whose butterflies are lazy too, get it as well.
     dc.lazy_out = pl.lazy && pl.g.logN > kSmallLogN && *std::min_element(pl.primes.begin(), pl.primes.end()) > (1u << 24);
     for (int j = 0; j < pl.K; ++j) {
         if (dc.lazy_out) {

@@ -2,8 +2,8 @@
 //
 // Reference counterpart: fherma_init / fherma_run / fherma_free,
 // solve.cu:710-1083.  The product is three to five launches on one stream:
-// decompose a and b (scaled), the transform chain (one launch where it fits the
-// GPU at once, else column pass, fused row pass, inverse column pass), CRT.  The
+// decompose a and b (scaled), the transform chain (one launch for few enough
+// blocks, else column pass, fused row pass, inverse column pass), CRT.  The
 // host path stages a caller's pageable buffers through pinned memory in chunks
 // so the copies overlap the host-side memcpys.
 #include "engine.h"

@@ -62,8 +62,8 @@ void build_row_tables(const DevPoint& d, uint2* out, cudaStream_t st);
 
 // The whole chain in one launch (ntt_fused.cu): N = 2^8 .. 2^11 in a block per
 // prime (products and forward transforms), N = 2^12 .. 2^15 in a cluster per
-// prime (products whose clusters are all resident at once).  N = 2^8 .. 2^10 read tables of their own, K x N pairs from
-// build_whole_tables (DevPoint::row_tw).
+// prime (products, up to four CTAs per SM).  N = 2^8 .. 2^10 read tables of
+// their own, K x N pairs from build_whole_tables (DevPoint::row_tw).
 bool ntt_fused_ok(const DevPoint& d, int mode, int sms);
 void launch_ntt_fused(const DevPoint& d, uint32_t* A, uint32_t* B, int mode, int sms, cudaStream_t st);
 void build_whole_tables(const DevPoint& d, uint2* out, cudaStream_t st);
@@ -125,7 +125,7 @@ struct DecConsts {
     const uint8_t* img[2];      // device copies of the plan's wide images, operands a and b
     uint32_t chunks;            // chunks of 4 piece primes (16 piece GEMM columns)
     uint32_t piece;             // primes per fold warp and chunk: 2, 4 .. 16
-    uint32_t lazy_out;          // 1: residues below 4p (congruent), for lazy first butterflies
+    uint32_t lazy_out;          // 1: residues below 2p (congruent), for lazy first butterflies
 };
 // Few tiles leave SMs idle and a CTA alone with all of a tile's primes: with
 // primes enough each tile is cut into the most parts the SMs take, a run of 4

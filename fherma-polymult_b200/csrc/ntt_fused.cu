@@ -1,7 +1,8 @@
-// The product's whole transform chain in one launch, for N = 2^8 .. 2^15 while
-// it fits the GPU at once.  A product of these sizes is a chain of short launches, and what it costs is
-// their number: three passes of a microsecond or two of work each, every one
-// behind the start, the first loads and the last stores of a launch of its own.
+// The product's whole transform chain in one launch, for N = 2^8 .. 2^15 where
+// that is the faster (ntt_fused_ok).  A product of these sizes is a chain of
+// short launches, and what it costs is their number: three passes of a
+// microsecond or two of work each, every one behind the start, the first loads
+// and the last stores of a launch of its own.
 //
 //   * N = 2^12 .. 2^15 (rows of S = 64 .. 512, R = 64): a cluster of N / 2048
 //     CTAs per prime.  Each holds one 2048-element tile of A and of B: it runs
@@ -12,9 +13,10 @@
 //     cross memory once in and once out (12 K N bytes instead of 28).
 //   * N = 2^8 .. 2^11 (R = 1): one CTA per prime holds both operands, one
 //     group of threads each for the forward rounds; the group of A multiplies
-//     and goes back.  (us, against one butterfly a thread with a barrier and a
-//     twiddle load from L2 at every stage: N = 256 K = 6 6.3 -> 1.9, N = 1024
-//     K = 59 10.9 -> 2.9; N = 2048 K = 10, a row pass with one group, 3.9 -> 3.7.)
+//     and goes back.  (us in a graph, against one butterfly a thread with a
+//     barrier and a twiddle load from L2 at every stage: N = 256 K = 6 6.1 -> 1.7,
+//     N = 1024 K = 59 10.7 -> 3.1; N = 2048 K = 138, a row pass with one group,
+//     8.0 -> 4.3.)
 //
 // What bounds both is latency: the rounds' serial chain at one block's warps,
 // then the exchanges.
@@ -278,8 +280,8 @@ __global__ void __launch_bounds__(2 * WholeGeom<LOGN>::T) k_ntt_whole(DevPoint d
     const RowTable<LOGN, 0, false, 0> fw{tf};
     const RowTable<LOGN, 0, true, 0> iw{tf};
     __syncthreads();
-    // (After the wait, as in the cluster kernel: N = 1024 K = 59 12.2 us a
-    // product for 11.7.)
+    // (After the wait, as in the cluster kernel: let in before it the CRT's
+    // blocks took N = 1024 K = 59 from 11.7 to 12.2 us a product.)
     pdl_wait();
     pdl_launch_dependents();
     uint32_t v[1][E];
@@ -540,15 +542,19 @@ void build_whole_tables(const DevPoint& d, uint2* out, cudaStream_t st) {
     check(cudaGetLastError(), "transform tables launch");
 }
 
-// Clusters while all their CTAs are resident at once, four on an SM (592 on 148
-// SMs): N = 4096 and 8192 at any K, 16384 up to K = 74, 32768 up to K = 37.  Past
-// one wave a cluster waits for as many free places as it has CTAs, and four
-// blocks an SM hold fewer warps than the separate passes (us, one launch
-// against three, B200):
-//   N = 4096   K = 19   5.3 |  7.7   K = 60   6.7 | 12.5   K = 138  8.9 | 16.3
-//   N = 8192   K = 10   6.5 |  8.0   K = 60  10.8 | 14.5   K = 139 12.2 | 18.3
-//   N = 16384  K = 36  11.7 | 17.2   K = 72  16.5 | 18.5   K = 139 26.5 | 23.4
-//   N = 32768  K = 19  13.1 | 18.5   K = 36  17.1 | 19.1   K = 60  26.8 | 23.7
+// Clusters up to four CTAs per SM in all (592 on 148 SMs: N = 4096 and 8192 at
+// any K, 16384 up to K = 74, 32768 up to K = 37), the measured crossover.  A
+// cluster lies within a group of SMs that share a network, so fewer are
+// resident at once than four CTAs an SM would give: 296, 142, 71 and 31 of
+// them for N = 4096 .. 32768 (cudaOccupancyMaxActiveClusters).  The last few wait
+// for a whole cluster's places, and still the one launch is no slower up to the
+// line (product us in a graph, one launch | three, B200):
+//   N = 4096   K = 60  15.5 | 21.7   K = 138 23.2 | 30.4
+//   N = 8192   K = 60  18.9 | 23.2   K = 130 30.2 | 35.5
+//   N = 16384  K = 36  22.1 | 24.6   K = 71  27.7 | 31.7   K = 72  31.1 | 31.4   K = 74  30.6 | 31.2
+//   N = 32768  K = 19  22.9 | 25.3   K = 31  26.3 | 30.3   K = 32  29.0 | 30.8   K = 37  31.2 | 31.9
+// and past it the separate passes, which hold more warps an SM, win (transform
+// alone: N = 16384 K = 139 26.5 | 23.4, N = 32768 K = 60 26.8 | 23.7).
 bool ntt_fused_ok(const DevPoint& d, int mode, int sms) {
     if (d.logN >= kWholeMinLogN && d.logN <= 11) return mode == kRowProduct || mode == kRowForward;
     if (mode != kRowProduct || d.logR != 6 || d.logS < 6 || d.logS > 9) return false;
