@@ -615,24 +615,21 @@ __global__ void __launch_bounds__(256, 6) k_ntt_col_inv_mixed(const __grid_const
     }
 }
 
-// Shared memory: the tables barriers' 32 bytes, aligned, past `bytes` of tiles
-// and tables, which a 256-thread tile has to itself and two 128-thread tiles
-// halve (mixed_row_bytes).  Block b of item i: tile local(b) (one per block) or
-// tiles 2 local(b) + half (two per block), tile = (prime, row block).
+// Shared memory: `bytes` of tiles and tables, which a 256-thread tile has to
+// itself and two 128-thread tiles halve (mixed_row_bytes), then the tables
+// barriers, one for 256-thread tiles and one per half.  Block b of item i: tile
+// local(b) (one per block) or tiles 2 local(b) + half (two per block), tile =
+// (prime, row block).
 template <bool LAZY>
 __global__ void __launch_bounds__(256, 3) k_ntt_row_mixed(const __grid_constant__ GroupTable t, uint32_t bytes) {
     extern __shared__ __align__(1024) uint32_t smem[];
-    uint8_t* base = reinterpret_cast<uint8_t*>(smem);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(base + bytes);
-    uint64_t* tbar[2] = {bars, bars + 2};
+    uint64_t* const bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(smem) + bytes);
     if (threadIdx.x == 0) {
-        tc::mbar_init(tbar[0], 1);
-        tc::mbar_init(tbar[1], 1);
+        for (int i = 0; i < 3; ++i) tc::mbar_init(bars + i, 1);
         tc::fence_mbar_init();
     }
     __syncthreads();
-    uint32_t uses[2] = {0, 0};   // every thread counts both regions' uses
-    const uint32_t half = threadIdx.x >> 7;
+    uint32_t phase = 0;   // bit 0: of the first barrier's next use, bit 1: of the other two's
     for (uint32_t b = blockIdx.x; b < t.total; b += gridDim.x) {
         if (b != blockIdx.x) {
             // Tiles of different row lengths lie differently: the bulk copies of
@@ -649,15 +646,13 @@ __global__ void __launch_bounds__(256, 3) k_ntt_row_mixed(const __grid_constant_
             const uint32_t per = row_blocks<LS>(6);
             if constexpr (row_threads<LS>() == 256) {
                 row_body<LS, LAZY, BlockTeam>(it.d, it.A, it.B, kRowProduct, it.j0 + local / per, local % per,
-                                              uses[0] & 1, smem, tbar[0]);
-                ++uses[0];
+                                              phase & 1u, smem, bars);
+                phase ^= 1u;
             } else {
-                const uint32_t tile = 2 * local + half;
+                const uint32_t half = threadIdx.x >> 7, tile = 2 * local + half;
                 row_body<LS, LAZY, HalfTeam>(it.d, it.A, it.B, kRowProduct, it.j0 + tile / per, tile % per,
-                                             uses[half] & 1, reinterpret_cast<uint32_t*>(base + half * (bytes / 2)),
-                                             tbar[half]);
-                ++uses[0];
-                ++uses[1];
+                                             phase >> 1, smem + half * (bytes / 8), bars + 1 + half);
+                phase ^= 2u;
             }
         });
     }
