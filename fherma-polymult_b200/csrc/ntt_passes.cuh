@@ -163,7 +163,7 @@ constexpr size_t row_bar_offset() {
 // 2^max_log_s: room for one 256-thread tile or, in halves, two 128-thread ones.
 // (With a region the size of the largest tile for each half, S = 2048 took 130
 // KB, one block an SM: N = 2^17, 2^16, 2^14 and 2^13 in one batch 295 us, with
-// this 262; before there were such tiles 266.)
+// this 262 at the same code otherwise.)
 constexpr uint32_t mixed_row_bytes(uint32_t max_log_s) {
     const int threads[6] = {row_threads<6>(), row_threads<7>(), row_threads<8>(),
                             row_threads<9>(), row_threads<10>(), row_threads<11>()};
