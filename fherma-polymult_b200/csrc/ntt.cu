@@ -1,6 +1,7 @@
 // Negacyclic NTT kernels: the column pass, the fused row pass (forward rows of
 // both operands, pointwise product, inverse rows) and the inverse column pass of
-// the four-step transform, plus a one-block-per-prime kernel for N <= 1024.
+// the four-step transform, plus a one-block-per-prime kernel for N < 256 (the
+// one-launch transforms of N = 2^8 .. 2^15 are in ntt_fused.cu).
 //
 // Reference counterparts (Akram275/fherma-polymult): k_ntt_cols solve.cu:130-166,
 // k_ntt_rows_mul solve.cu:195-233, with the stage structure of

@@ -1,5 +1,5 @@
-// Register-blocked NTT rounds on a shared-memory tile of 2^BITS elements (2048
-// but for the transforms of N <= 1024, whose tile is the whole polynomial).
+// Register-blocked NTT rounds on a shared-memory tile of 2^BITS elements (2048,
+// but 4096 for rows of 2048 and the whole polynomial for N <= 1024).
 //
 // A tile holds 2048 / 2^NSUB independent sub-transforms of 2^NSUB elements.  The
 // tile index i carries the position x inside a sub-transform in bits
